@@ -178,20 +178,20 @@ int sqb_set_launch(sqb_ctx *ctx, int ctas_per_sm, int cols_per_thread);
  * projectors per type.  SQB_KERNEL_PLANE: the plane-streaming kernel with
  * per-window box lists, any system.  SQB_KERNEL_AUTO (default): the sweep
  * kernel where it covers the system.  Results agree to rounding.  The nonlocal
- * forces, the adjoint, sqb_moments_at, sqb_hsub_times_vec and
- * sqb_lanczos_moments_noalloc run the plane-streaming kernel.  No counterpart
- * in the reference. */
+ * forces and the adjoint follow the same choice; sqb_moments_at,
+ * sqb_hsub_times_vec and sqb_lanczos_moments_noalloc run the plane-streaming
+ * kernel.  No counterpart in the reference. */
 #define SQB_KERNEL_AUTO 0
 #define SQB_KERNEL_PLANE 1
 #define SQB_KERNEL_SWEEP 2
 int sqb_set_node_kernel(sqb_ctx *ctx, int kernel);
-/* Window rows per thread of the sweep kernel: 2 (one column and two rows per
- * thread, the default), 3 (fewer threads, more registers each; windows up to
- * 33 wide), or 0 for the default.  Results agree to rounding (the block
+/* Tile of the sweep kernel's threads: 0 or 2 the default one (a pair of window
+ * columns and one row per thread), 3 a pair of columns and three rows (fewer
+ * threads, more registers each; windows up to 33 wide).  Results agree to rounding (the block
  * reductions sum in another order). */
 int sqb_set_sweep_rows(sqb_ctx *ctx, int rows);
-/* Times the SQ node work on the sweep kernel with two and with three rows
- * per thread on `sample` evenly spaced nodes (0: two per SM), keeps the
+/* Times the SQ node work on the sweep kernel with the default tile (2) and
+ * with three rows per thread (3) on `sample` evenly spaced nodes (0: two per SM), keeps the
  * faster for the context; *rows the choice, ms[2] the times (-1 where a
  * variant does not apply).  SQB_ERR_UNSUPPORTED when the sweep kernel does
  * not cover the context. */

@@ -43,6 +43,8 @@ struct sqb_ctx {
   void *allreduce_user = nullptr;
 
   double *d_veff64 = nullptr;
+  double *d_veffp = nullptr;  // the same in rows of exp values (the sweep kernel's)
+  int exp = 0;                // row pitch of the sweep kernel's fields: even, at least ex + 1
   bool have_veff = false;
 
   int n_typ = 0, n_rep = 0, n_atm = 0;
@@ -77,6 +79,7 @@ struct sqb_ctx {
   int4 *d_rep_box = nullptr;
   int *d_rep_gpb = nullptr;
   int *d_rep_atom_l = nullptr;  // global atom of each replica of d_rep_box
+  long long *d_rep_off_l = nullptr;  // and its offset in the padded tables
   bool have_atoms = false, have_proj = false;
 
   unsigned char *d_scratch = nullptr;
@@ -278,9 +281,8 @@ int run_nodes(sqb_ctx *c, NodeArgs &a, const int *d_list, int count) {
 
 // Layered projector fields of the sweep kernel: the replica balls with
 // projectors, as boxes on the extended grid (the block with its nloc halo),
-// split greedily in replica order into layers whose balls neither overlap nor
-// touch along z (a gap of at least one plane where their x-y footprints
-// overlap).  The sweep kernel covers the context when four layers suffice,
+// split into layers whose balls neither overlap nor touch along z (a gap of at
+// least one plane where their x-y footprints overlap).  The sweep kernel covers the context when four layers suffice,
 // every type has at most three projectors, the ids fit 16 bits and the
 // block's shared memory holds the kernel's working set; otherwise the
 // plane-streaming kernel runs.
@@ -310,26 +312,56 @@ int ensure_layers(sqb_ctx *c) {
     boxes.push_back(b);
     pmax = std::max(pmax, np);
   }
-  std::vector<std::vector<int>> layers;
-  std::vector<int> layer_of(boxes.size());
-  for (size_t i = 0; i < boxes.size(); i++) {
-    const Box &b = boxes[i];
-    int k = 0;
-    for (; k < (int)layers.size(); k++) {
-      bool clash = false;
-      for (int j : layers[k]) {
-        const Box &o = boxes[j];
-        if (b.lo[0] <= o.hi[0] && o.lo[0] <= b.hi[0] && b.lo[1] <= o.hi[1] && o.lo[1] <= b.hi[1] &&
-            b.lo[2] <= o.hi[2] + 1 && o.lo[2] <= b.hi[2] + 1) {
-          clash = true;
-          break;
+  // Balls of one layer must not overlap, nor touch along z (a column's flush
+  // at a ball's last plane needs its own slot).
+  const int nb = (int)boxes.size();
+  std::vector<std::vector<int>> clash(nb);
+  for (int i = 0; i < nb; i++)
+    for (int j = 0; j < i; j++) {
+      const Box &b = boxes[i], &o = boxes[j];
+      if (b.lo[0] <= o.hi[0] && o.lo[0] <= b.hi[0] && b.lo[1] <= o.hi[1] && o.lo[1] <= b.hi[1] &&
+          b.lo[2] <= o.hi[2] + 1 && o.lo[2] <= b.hi[2] + 1) {
+        clash[i].push_back(j);
+        clash[j].push_back(i);
+      }
+    }
+  std::vector<int> layer_of(nb, -1);
+  auto first_free = [&](int i) {
+    for (int k = 0;; k++) {
+      bool used = false;
+      for (int j : clash[i]) used = used || layer_of[j] == k;
+      if (!used) return k;
+    }
+  };
+  int n_layers = 0;
+  for (int i = 0; i < nb; i++) n_layers = std::max(n_layers, (layer_of[i] = first_free(i)) + 1);
+  if (n_layers > LAYERS) {
+    // First fit in replica order can start two far-apart balls on layers that
+    // their common neighbours then cannot share.  Colouring next the ball whose
+    // neighbours already use the most layers (DSATUR, Brelaz 1979) finds the
+    // four sublattices of a displaced FCC cell: of the 108-atom cell's blocks
+    // one in three failed by first fit, of 64-atom LiH every one, and then ran
+    // on the plane-streaming kernel at less than half the speed.
+    std::fill(layer_of.begin(), layer_of.end(), -1);
+    std::vector<std::vector<char>> seen(nb);  // layers among a ball's neighbours
+    std::vector<int> sat(nb, 0);
+    n_layers = 0;
+    for (int step = 0; step < nb; step++) {
+      int best = -1;
+      for (int i = 0; i < nb; i++)
+        if (layer_of[i] < 0 && (best < 0 || sat[i] > sat[best] ||
+                                (sat[i] == sat[best] && clash[i].size() > clash[best].size())))
+          best = i;
+      const int k = layer_of[best] = first_free(best);
+      n_layers = std::max(n_layers, k + 1);
+      for (int j : clash[best]) {
+        if ((int)seen[j].size() <= k) seen[j].resize(k + 1, 0);
+        if (!seen[j][k]) {
+          seen[j][k] = 1;
+          sat[j]++;
         }
       }
-      if (!clash) break;
     }
-    if (k == (int)layers.size()) layers.emplace_back();
-    layers[k].push_back((int)i);
-    layer_of[i] = k;
   }
   std::vector<int4> box4(std::max<size_t>(boxes.size(), 1));
   std::vector<int> gpb(std::max<size_t>(boxes.size(), 1));
@@ -343,13 +375,12 @@ int ensure_layers(sqb_ctx *c) {
   const int pm = pmax <= 1 ? 1 : 3;
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  const long long evol_all = (long long)c->ex * c->ey * c->ez;
-  const bool usable = (int)layers.size() <= LAYERS && pmax <= LAY_PMAX && ngp + pm < 65535 &&
-                      evol_all * LAYERS * LAY_PMAX < (1LL << 31) &&
-                      sweep_rows_supported(c->n, 2) && sweep_smem(c->n, pm, ngp, 2) <= (size_t)optin &&
+  const long long evol = (long long)c->exp * c->ey * c->ez;
+  const bool usable = n_layers <= LAYERS && pmax <= LAY_PMAX && ngp + pm < 65535 &&
+                      evol * LAYERS * LAY_PMAX < (1LL << 31) &&
+                      sweep_rows_supported(c->n, 1) && sweep_smem(c->n, pm, ngp, 1) <= (size_t)optin &&
                       c->n_typ < 256;
   if (!usable) return SQB_OK;
-  const long long evol = (long long)c->ex * c->ey * c->ez;
   c->n_gproj = ngp;
   c->lay_pmax = pm;
   c->n_lrep = (int)boxes.size();
@@ -375,7 +406,7 @@ int ensure_layers(sqb_ctx *c) {
   CK(cudaMalloc((void **)&d_off, off.size() * sizeof(long long)));
   CK(cudaMemcpy(d_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice));
   const cudaError_t e = launch_fill_layers((int)boxes.size(), c->d_rep_box, c->d_rep_gpb, c->d_typ_nlocc, d_off,
-                                           c->d_tab64, c->ex, c->ey, c->ez, pm, ngp, c->d_lay_id, c->d_lay_chi,
+                                           c->d_tab64, c->ex, c->ey, c->ez, c->exp, pm, ngp, c->d_lay_id, c->d_lay_chi,
                                            c->stream);
   const cudaError_t e2 = cudaStreamSynchronize(c->stream);
   cudaFree(d_off);
@@ -410,36 +441,32 @@ int ensure_sweep_scratch(sqb_ctx *c, int grid, size_t *stride) {
   return SQB_OK;
 }
 
-// Window rows per sweep-kernel thread: the requested count where the kernel
-// covers it (sqb_set_sweep_rows, sqb_autotune_sweep), else 2.  (Three rows
-// give fewer threads more registers; measured on the B200 they were slower
-// also where the fields carry three projectors per slot: c3 FP64 199 against
-// 167 ms on a 296-node sample, forces 34.8 against 27.9 s.)
+// Window rows per sweep-kernel thread: three where asked for (sqb_set_sweep_rows,
+// sqb_autotune_sweep) and covered, else the default tile's.
 int sweep_rows(const sqb_ctx *c) {
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  auto fits = [&](int ry) {
-    return sweep_rows_supported(c->n, ry) && sweep_smem(c->n, c->lay_pmax, c->n_gproj, ry) <= (size_t)optin;
-  };
-  if (c->sweep_ry && fits(c->sweep_ry)) return c->sweep_ry;
-  return 2;
+  if (c->sweep_ry == 3 && sweep_rows_supported(c->n, 3) &&
+      sweep_smem(c->n, c->lay_pmax, c->n_gproj, 3) <= (size_t)optin)
+    return 3;
+  return 1;
 }
 
 // The context's part of a sweep-kernel launch (grid, fields, replicas, queue).
-void fill_sweep_args(sqb_ctx *c, const int *d_list, int count, size_t stride, SweepArgs &s) {
+void fill_sweep_args(sqb_ctx *c, const int *d_list, int count, SweepArgs &s) {
   std::memset(&s, 0, sizeof(s));
   s.n = c->n;
   s.nloc = c->g.nloc;
   s.npl = c->g.npl;
   for (int d = 0; d < 3; d++) s.np[d] = c->g.np[d];
-  s.ex = c->ex;
+  s.ex = c->exp;
   s.ey = c->ey;
-  s.evol = (long long)c->ex * c->ey * c->ez;
+  s.evol = (long long)c->exp * c->ey * c->ez;
   s.h3 = c->h3;
   s.lanczos_tol = c->g.lanczos_tol;
   for (int k = 0; k <= FDN; k++) s.coeff_lap[k] = c->g.coeff_lap[k];
   for (int k = 0; k <= FDN; k++) s.coeff_grad[k] = c->g.coeff_grad[k];
-  s.veff64 = c->d_veff64;
+  s.veff64 = c->d_veffp;
   s.n_gproj = c->n_gproj;
   s.pmax = c->lay_pmax;
   s.lay_id = c->d_lay_id;
@@ -454,11 +481,28 @@ void fill_sweep_args(sqb_ctx *c, const int *d_list, int count, size_t stride, Sw
   s.n_list = count;
   s.counter = c->d_counter;
   s.status = c->d_status;
-  s.scratch = c->d_scratch;
-  s.scratch_stride = stride;
   s.ry = sweep_rows(c);
   s.nsweep = sweep_threads(c->n, s.ry);
   s.proj_points = c->d_proj_points;
+}
+
+// CTAs of a sweep-kernel launch (all resident: the queue hands out nodes) and
+// their scratch.  Small windows keep several CTAs on an SM, each with its own
+// node, so that one node's barriers and serial parts overlap with others.
+int sweep_grid(sqb_ctx *c, int per_sm, SweepArgs &s, int *grid) {
+  *grid = std::max(1, std::min(c->sms * per_sm, s.n_list));
+  const int rc = ensure_sweep_scratch(c, *grid, &s.scratch_stride);
+  s.scratch = c->d_scratch;
+  return rc;
+}
+
+// Arguments, grid and scratch of an SQ launch on the sweep kernel.
+int prepare_sq_sweep(sqb_ctx *c, const NodeArgs &a, const int *d_list, int count, SweepArgs &s, int *grid) {
+  fill_sweep_args(c, d_list, count, s);
+  s.form = a.lq ? 2 : (a.mixed ? 1 : 0);
+  int per_sm = 0;
+  CK(sweep_per_sm(s, &per_sm));
+  return sweep_grid(c, per_sm, s, grid);
 }
 
 // Lanczos bounds and Chebyshev moments (MODE_SQ) of `count` nodes of d_list
@@ -470,15 +514,10 @@ int run_sq_nodes(sqb_ctx *c, NodeArgs &a, const int *d_list, int count) {
   if (rc) return rc;
   c->stats.node_kernel = sw ? SQB_KERNEL_SWEEP : SQB_KERNEL_PLANE;
   if (!sw) return run_nodes(c, a, d_list, count);
-  int grid = c->sms;
-  if (grid > count) grid = count;
-  if (grid < 1) grid = 1;
-  size_t stride = 0;
-  rc = ensure_sweep_scratch(c, grid, &stride);
-  if (rc) return rc;
   SweepArgs s;
-  fill_sweep_args(c, d_list, count, stride, s);
-  s.form = a.lq ? 2 : (a.mixed ? 1 : 0);
+  int grid = 0;
+  rc = prepare_sq_sweep(c, a, d_list, count, s, &grid);
+  if (rc) return rc;
   s.lanczos_tol = a.lanczos_tol;
   s.lz_chk = a.lz_chk;
   s.chi = a.chi;
@@ -747,8 +786,7 @@ int sqb_create(const sqb_grid *grid, int device, sqb_ctx **out) {
   CK(cudaEventCreate(&c->ev1));
   CK(cudaEventCreateWithFlags(&c->ev_order, cudaEventDisableTiming));
   CK(node_kernel_setup(c->n));
-  CK(sweep_setup(c->n));
-  CK(sweep_forces_setup(c->n));
+  c->exp = (c->ex + 2) & ~1;
   const size_t N = c->nnode, K = g.npl + 1;
   CK(dalloc(&c->d_counter, 1));
   CK(dalloc(&c->d_status, 1));
@@ -788,7 +826,7 @@ int sqb_destroy(sqb_ctx *c) {
   if (!c) return SQB_OK;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  void *ptrs[] = {c->d_lay_id, c->d_lay_chi, c->d_rep_box, c->d_rep_gpb, c->d_rep_atom_l, c->d_veff64, c->d_rep_nn, c->d_rep_atom, c->d_rep_off, c->d_typ_tab,
+  void *ptrs[] = {c->d_lay_id, c->d_lay_chi, c->d_rep_box, c->d_rep_gpb, c->d_rep_atom_l, c->d_rep_off_l, c->d_veff64, c->d_veffp, c->d_rep_nn, c->d_rep_atom, c->d_rep_off, c->d_typ_tab,
                   c->d_typ_nlocc, c->d_typ_nproj, c->d_typ_lmax, c->d_typ_lloc, c->d_typ_size, c->d_proj_denom,
                   c->d_tables, c->d_rep_xyz, c->d_rep_off_ref, c->d_vjp, c->d_vjp_at, c->d_dtab, c->d_tab64, c->d_scratch, c->d_counter, c->d_nodes,
                   c->d_status, c->d_iters, c->d_proj_points, c->d_chi, c->d_zee, c->d_rho_pj, c->d_lmin,
@@ -842,6 +880,18 @@ int sqb_set_launch(sqb_ctx *c, int ctas_per_sm, int cols_per_thread) {
   return SQB_OK;
 }
 
+// The padded copy of Veff the sweep kernel reads (pad values zero).
+static int pad_veff(sqb_ctx *c) {
+  const size_t rows = (size_t)c->ey * c->ez;
+  if (!c->d_veffp) {
+    CK(dalloc(&c->d_veffp, rows * c->exp));
+    CK(cudaMemsetAsync(c->d_veffp, 0, rows * c->exp * sizeof(double), c->stream));
+  }
+  CK(cudaMemcpy2DAsync(c->d_veffp, c->exp * sizeof(double), c->d_veff64, c->ex * sizeof(double),
+                       c->ex * sizeof(double), rows, cudaMemcpyDeviceToDevice, c->stream));
+  return SQB_OK;
+}
+
 int sqb_set_veff(sqb_ctx *c, const double *veff_ext) {
   if (!c || !veff_ext) return SQB_ERR_ARG;
   cudaSetDevice(c->device);
@@ -850,6 +900,7 @@ int sqb_set_veff(sqb_ctx *c, const double *veff_ext) {
     if (!std::isfinite(veff_ext[i])) return SQB_ERR_NONFINITE;
   if (!c->d_veff64) CK(dalloc(&c->d_veff64, n));
   CK(cudaMemcpyAsync(c->d_veff64, veff_ext, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  if (const int rc = pad_veff(c)) return rc;
   CK(cudaStreamSynchronize(c->stream));
   c->have_veff = true;
   c->have_moments = false;
@@ -867,6 +918,7 @@ int sqb_set_veff_device(sqb_ctx *c, const double *veff_ext) {
   CK(cudaEventRecord(c->ev_order, cudaStreamLegacy));
   CK(cudaStreamWaitEvent(c->stream, c->ev_order, 0));
   CK(cudaMemcpyAsync(c->d_veff64, veff_ext, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+  if (const int rc = pad_veff(c)) return rc;
   CK(cudaStreamSynchronize(c->stream));
   c->have_veff = true;
   c->have_moments = false;
@@ -1372,11 +1424,6 @@ int sqb_spectral_quadrature(sqb_ctx *c, int scf_iter, double *lambda_f, double *
 // several ranks go through the host) and without the defect check.
 static int build_step_graph(sqb_ctx *c) {
   if (!c->d_fermi) CK(cudaMalloc((void **)&c->d_fermi, sizeof(FermiDev)));
-  {  // allocate what the captured launches use (no allocation inside a capture)
-    size_t stride = 0;
-    const int rc0 = ensure_sweep_scratch(c, std::max(1, std::min(c->sms, c->nnode)), &stride);
-    if (rc0) return rc0;
-  }
   NodeArgs a;
   fill_node_args(c, a);
   a.mode = MODE_SQ;
@@ -1386,6 +1433,12 @@ static int build_step_graph(sqb_ctx *c) {
   a.lmin = c->d_lmin;
   a.lmax = c->d_lmax;
   a.lanczos_iters = c->d_iters;
+  {  // allocate what the captured launches use (no allocation inside a capture)
+    SweepArgs s;
+    int grid = 0;
+    const int rc0 = prepare_sq_sweep(c, a, c->d_nodes, c->nnode, s, &grid);
+    if (rc0) return rc0;
+  }
   FermiArgs fa = fermi_args(c);
   fa.lam_dev = &c->d_fermi->x;
   FermiArgs fd = fermi_args(c);
@@ -1938,12 +1991,13 @@ static int forces_nonlocal(sqb_ctx *c, const double *chi, const double *zee, con
   c->stats.kernel_launches = 0;
   c->stats.node_kernel = sw ? SQB_KERNEL_SWEEP : SQB_KERNEL_PLANE;
   if (sw) {
-    const int grid = std::max(1, std::min(c->sms, c->nnode));
-    size_t stride = 0;
-    rc = ensure_sweep_scratch(c, grid, &stride);
-    if (rc) return rc;
     SweepArgs s;
-    fill_sweep_args(c, c->d_nodes, c->nnode, stride, s);
+    fill_sweep_args(c, c->d_nodes, c->nnode, s);
+    const int single = c->precision == SQB_FP32_MIXED;
+    int per_sm = 0, grid = 0;
+    CK(sweep_forces_per_sm(s, single, &per_sm));
+    rc = sweep_grid(c, per_sm, s, &grid);
+    if (rc) return rc;
     s.chi = c->d_chi;
     s.zee = c->d_zee;
     s.ci = c->d_ci;
@@ -1952,7 +2006,7 @@ static int forces_nonlocal(sqb_ctx *c, const double *chi, const double *zee, con
     CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
     CK(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
     CK(cudaMemsetAsync(c->d_proj_points, 0, 3 * sizeof(unsigned long long), c->stream));
-    CK(launch_sweep_forces(s, c->precision == SQB_FP32_MIXED, grid, c->stream));
+    CK(launch_sweep_forces(s, single, grid, c->stream));
   } else {
     NodeArgs a;
     fill_node_args(c, a);

@@ -132,6 +132,9 @@ struct SweepArgs {
              // (FP32 Lanczos vectors, FP64 moments); 2: Lanczos quadrature
   int n, nloc, npl;
   int np[3];
+  // the extended grid of the fields and of veff64: rows of ex values, the block
+  // with its halo padded by at least one value to an even pitch, so that a
+  // 16-byte access at an even column stays inside its row
   int ex, ey;
   long long evol;  // ex * ey * ez
   double h3, lanczos_tol, lz_chk;
@@ -157,7 +160,7 @@ struct SweepArgs {
   unsigned char *scratch;
   size_t scratch_stride;  // bytes per CTA: three window vectors (FP64), then the flush buffer
   int nsweep;             // threads of the block (a multiple of 32)
-  int ry;                 // window rows per thread (2, or 3 up to 33-wide windows)
+  int ry;                 // window rows per thread (1, or 3 up to 33-wide windows)
   double *chi, *zee, *rho_pj, *lmin, *lmax;
   int *lanczos_iters;
   // ForcesNonLocal (sweep_force_kernel): bounds in chi, zee (inputs), the
@@ -176,16 +179,17 @@ int sweep_threads(int n, int ry);
 size_t sweep_smem(int n, int pmax, int n_gproj, int ry);
 bool sweep_rows_supported(int n, int ry);
 size_t sweep_scratch_bytes(int n, int pmax);  // scratch per CTA
-cudaError_t sweep_setup(int n);
+cudaError_t sweep_per_sm(const SweepArgs &a, int *per_sm);  // resident CTAs per SM of the launch's kernel
 cudaError_t launch_sweep(const SweepArgs &a, int grid, cudaStream_t s);
 // ForcesNonLocal on the sweep kernel (sqb_sweep_forces.cu); single: FP32
 // storage of the Chebyshev vectors (the FP32-mixed form), else FP64.
-cudaError_t sweep_forces_setup(int n);
+cudaError_t sweep_forces_per_sm(const SweepArgs &a, int single, int *per_sm);
 cudaError_t launch_sweep_forces(const SweepArgs &a, int single, int grid, cudaStream_t s);
 // Layered fields from the padded projector tables: ids and values of every
-// replica's ball on the extended grid (fields zeroed / set empty first).
+// replica's ball on the extended grid (ex x ey x ez points, rows of pitch
+// values; fields zeroed / set empty first).
 cudaError_t launch_fill_layers(int n_rep, const int4 *rep_box, const int *rep_gpb, const int *typ_nlocc,
-                               const long long *rep_off, const double *tab64, int ex, int ey, int ez, int pmax,
+                               const long long *rep_off, const double *tab64, int ex, int ey, int ez, int pitch, int pmax,
                                int n_gproj, unsigned long long *lay_id, double *lay_chi, cudaStream_t s);
 
 // Host-side launchers (sqb_node.cu).

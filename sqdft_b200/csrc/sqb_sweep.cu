@@ -10,9 +10,9 @@ namespace {
 // of the fields, and its first projector id into the point's id word.  The
 // balls of one layer do not overlap, so every field value has one writer.
 __global__ void fill_layers_kernel(int n_rep, const int4 *rep_box, const int *rep_gpb, const int *typ_nlocc,
-                                   const long long *rep_off, const double *tab64, int ex, int ey, int ez, int pmax,
+                                   const long long *rep_off, const double *tab64, int ex, int ey, int ez, int pitch, int pmax,
                                    unsigned short *lay_id16, double *lay_chi) {
-  const long long evol = (long long)ex * ey * ez;
+  const long long evol = (long long)pitch * ey * ez;
   for (int r = blockIdx.x; r < n_rep; r += gridDim.x) {
     const int4 b = rep_box[r];
     const int x0 = (short)(b.x & 0xffff), y0 = (short)(b.y & 0xffff), z0 = (short)(b.z & 0xffff);
@@ -24,7 +24,7 @@ __global__ void fill_layers_kernel(int n_rep, const int4 *rep_box, const int *re
       const int bx = i % Sd, by = (i / Sd) % Sd, bz = i / (Sd * Sd);
       const int X = x0 + bx, Yc = y0 + by, Z = z0 + bz;
       if (X < 0 || X >= ex || Yc < 0 || Yc >= ey || Z < 0 || Z >= ez) continue;
-      const long long g = ((long long)Z * ey + Yc) * ex + X;
+      const long long g = ((long long)Z * ey + Yc) * pitch + X;
       lay_id16[g * 4 + k] = (unsigned short)rep_gpb[r];
       for (int q = 0; q < np && q < pmax; q++)
         lay_chi[(long long)(k * pmax + q) * evol + g] = U[(long long)(q * Sd + bz) * sp2 + by * Sd + bx];
@@ -37,50 +37,24 @@ __global__ void fill_empty_kernel(unsigned long long *lay_id, long long evol, un
     lay_id[i] = empty;
 }
 
-// Launch bounds of the instantiations (the register budget per thread is
-// set by the warps per SM sub-partition).  Two rows per thread: windows up
-// to 31 wide run 512 threads (16 warps, 128 registers), 33 wide 576 (96), up
-// to 43 wide 1024.  Three rows per thread: up to 33 wide, 384 threads (12
-// warps, 168 registers), for fields whose many dot-product accumulators
-// spill at the smaller budgets.
-constexpr int MAXT_A = 512, MAXT_B = 576, MAXT_C = 1024, MAXT_R3 = 384;
-
-template <int PM, int FORM, int MAXT, int RY>
-cudaError_t set_attr(size_t smem) {
-  return cudaFuncSetAttribute(sweep::sweep_kernel<PM, FORM, MAXT, RY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem);
-}
-
 template <int PM, int FORM>
-cudaError_t launch_form(const SweepArgs &a, int grid, int threads, size_t smem, cudaStream_t s) {
-  if (a.ry == 3) {
-    if (threads > MAXT_R3) return cudaErrorInvalidConfiguration;
-    sweep::sweep_kernel<PM, FORM, MAXT_R3, 3><<<grid, threads, smem, s>>>(a);
-  } else if (threads <= MAXT_A) sweep::sweep_kernel<PM, FORM, MAXT_A, 2><<<grid, threads, smem, s>>>(a);
-  else if (threads <= MAXT_B) sweep::sweep_kernel<PM, FORM, MAXT_B, 2><<<grid, threads, smem, s>>>(a);
-  else if (threads <= MAXT_C) sweep::sweep_kernel<PM, FORM, MAXT_C, 2><<<grid, threads, smem, s>>>(a);
-  else return cudaErrorInvalidConfiguration;
-  return cudaGetLastError();
-}
+struct SqKernels {
+  template <int MAXT, int RY, int MINB>
+  static const void *get() {
+    return reinterpret_cast<const void *>(&sweep::sweep_kernel<PM, FORM, MAXT, RY, MINB>);
+  }
+};
 
-template <int PM>
-cudaError_t launch_pm(const SweepArgs &a, int grid, int threads, size_t smem, cudaStream_t s) {
-  if (a.form == 0) return launch_form<PM, 0>(a, grid, threads, smem, s);
-  if (a.form == 1) return launch_form<PM, 1>(a, grid, threads, smem, s);
-  return launch_form<PM, 2>(a, grid, threads, smem, s);
-}
-
-template <int PM>
-cudaError_t setup_pm(size_t smem) {
-  cudaError_t r[12] = {set_attr<PM, 0, MAXT_A, 2>(smem),  set_attr<PM, 1, MAXT_A, 2>(smem),
-                       set_attr<PM, 2, MAXT_A, 2>(smem),  set_attr<PM, 0, MAXT_B, 2>(smem),
-                       set_attr<PM, 1, MAXT_B, 2>(smem),  set_attr<PM, 2, MAXT_B, 2>(smem),
-                       set_attr<PM, 0, MAXT_C, 2>(smem),  set_attr<PM, 1, MAXT_C, 2>(smem),
-                       set_attr<PM, 2, MAXT_C, 2>(smem),  set_attr<PM, 0, MAXT_R3, 3>(smem),
-                       set_attr<PM, 1, MAXT_R3, 3>(smem), set_attr<PM, 2, MAXT_R3, 3>(smem)};
-  for (cudaError_t e : r)
-    if (e != cudaSuccess) return e;
-  return cudaSuccess;
+const void *sq_kernel(const SweepArgs &a) {
+  if (a.pmax == 1)
+    return a.form == 0   ? sweep::pick_tile<SqKernels<1, 0>>(a.n, a.ry)
+           : a.form == 1 ? sweep::pick_tile<SqKernels<1, 1>>(a.n, a.ry)
+                         : sweep::pick_tile<SqKernels<1, 2>>(a.n, a.ry);
+  if (a.pmax == 3)
+    return a.form == 0   ? sweep::pick_tile<SqKernels<3, 0>>(a.n, a.ry)
+           : a.form == 1 ? sweep::pick_tile<SqKernels<3, 1>>(a.n, a.ry)
+                         : sweep::pick_tile<SqKernels<3, 2>>(a.n, a.ry);
+  return nullptr;
 }
 
 }  // namespace
@@ -88,46 +62,48 @@ cudaError_t setup_pm(size_t smem) {
 int sweep_threads(int n, int ry) { return sweep::sweep_threads_of(n, ry); }
 
 bool sweep_rows_supported(int n, int ry) {
-  if (ry == 2) return sweep::sweep_threads_of(n, 2) <= MAXT_C;
-  if (ry == 3) return sweep::sweep_threads_of(n, 3) <= MAXT_R3;
-  return false;
+  return (ry == 1 && n <= sweep::TILE_N_MAX) || (ry == 3 && n <= sweep::TILE_N_ROWS3);
 }
 
 size_t sweep_smem(int n, int pmax, int n_gproj, int ry) {
-  const int nt = sweep::sweep_threads_of(n, ry);
-  return sweep::shared_fixed() + sweep::planes_bytes(n, ry) + sweep::ring_bytes(nt, pmax, ry) +
-         sweep::accw_bytes(nt, pmax, ry) + (((size_t)(n_gproj + pmax) * sizeof(double) + 127) & ~size_t(127));
+  return sweep::shared_fixed() + sweep::planes_bytes(n, ry) + sweep::ring_bytes(sweep::tile_bound(n, ry), ry) +
+         (((size_t)(n_gproj + pmax) * sizeof(double) + 127) & ~size_t(127));
 }
 
 size_t sweep_scratch_bytes(int n, int pmax) {
-  const size_t nw = (size_t)n * n * n;
-  return ((3 * nw + sweep::flush_doubles(n, pmax)) * sizeof(double) + 255) & ~size_t(255);
+  return ((3 * sweep::vec_points(n) + sweep::flush_doubles(n, pmax)) * sizeof(double) + 255) & ~size_t(255);
 }
 
-cudaError_t sweep_setup(int n) {
-  (void)n;
-  int dev = 0, optin = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e != cudaSuccess) return e;
-  e = setup_pm<1>((size_t)optin);
-  if (e == cudaSuccess) e = setup_pm<3>((size_t)optin);
+namespace sweep {
+
+cudaError_t tile_setup(const void *kernel, const SweepArgs &a, int *per_sm) {
+  if (kernel == nullptr || a.n > MAXN || sweep_threads_of(a.n, a.ry) != a.nsweep) return cudaErrorInvalidConfiguration;
+  const size_t smem = sweep_smem(a.n, a.pmax, a.n_gproj, a.ry);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && per_sm) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, a.nsweep, smem);
+    if (e == cudaSuccess && *per_sm < 1) e = cudaErrorInvalidConfiguration;
+  }
   return e;
 }
 
+}  // namespace sweep
+
+cudaError_t sweep_per_sm(const SweepArgs &a, int *per_sm) { return sweep::tile_setup(sq_kernel(a), a, per_sm); }
+
 cudaError_t launch_sweep(const SweepArgs &a, int grid, cudaStream_t s) {
-  const int threads = sweep_threads(a.n, a.ry);
-  if (a.n > MAXN || !sweep_rows_supported(a.n, a.ry) || threads != a.nsweep) return cudaErrorInvalidConfiguration;
-  const size_t smem = sweep_smem(a.n, a.pmax, a.n_gproj, a.ry);
-  if (a.pmax == 1) return launch_pm<1>(a, grid, threads, smem, s);
-  if (a.pmax == 3) return launch_pm<3>(a, grid, threads, smem, s);
-  return cudaErrorInvalidValue;
+  const void *kernel = sq_kernel(a);
+  cudaError_t e = sweep::tile_setup(kernel, a, nullptr);
+  if (e != cudaSuccess) return e;
+  SweepArgs args = a;
+  void *argv[] = {&args};
+  return cudaLaunchKernel(kernel, dim3(grid), dim3(a.nsweep), argv, sweep_smem(a.n, a.pmax, a.n_gproj, a.ry), s);
 }
 
 cudaError_t launch_fill_layers(int n_rep, const int4 *rep_box, const int *rep_gpb, const int *typ_nlocc,
-                               const long long *rep_off, const double *tab64, int ex, int ey, int ez, int pmax,
+                               const long long *rep_off, const double *tab64, int ex, int ey, int ez, int pitch, int pmax,
                                int n_gproj, unsigned long long *lay_id, double *lay_chi, cudaStream_t s) {
-  const long long evol = (long long)ex * ey * ez;
+  const long long evol = (long long)pitch * ey * ez;
   cudaError_t e = cudaMemsetAsync(lay_chi, 0, (size_t)LAYERS * pmax * evol * sizeof(double), s);
   if (e != cudaSuccess) return e;
   const unsigned long long empty = 0x0001000100010001ull * (unsigned long long)n_gproj;
@@ -135,7 +111,7 @@ cudaError_t launch_fill_layers(int n_rep, const int4 *rep_box, const int *rep_gp
   e = cudaGetLastError();
   if (e != cudaSuccess || n_rep == 0) return e;
   fill_layers_kernel<<<n_rep < 4096 ? n_rep : 4096, 256, 0, s>>>(n_rep, rep_box, rep_gpb, typ_nlocc, rep_off, tab64,
-                                                                  ex, ey, ez, pmax,
+                                                                  ex, ey, ez, pitch, pmax,
                                                                   reinterpret_cast<unsigned short *>(lay_id), lay_chi);
   return cudaGetLastError();
 }

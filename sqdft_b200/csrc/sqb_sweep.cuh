@@ -7,15 +7,16 @@
 // matvec H v = -1/2 Lap_h v + Veff v + Vnl v on a node's (2nloc+1)^3 window
 // (HsubTimesVec sq.cpp:838-929, VnlocsubTimesVec nonlocal.cpp:20-215; v zero
 // outside the window) is one sweep over the window's z-planes:
-//   * each thread owns one window column x and RY adjacent rows y; it writes
-//     its centre values into a shared-memory plane with a zero halo of 6, so
-//     the x and y neighbours are unconditional loads (the window truncation
-//     falls out of the halo); the RY rows share their y-arm loads;
+//   * each thread owns a pair of window columns x and RY adjacent rows y; it
+//     writes its centre values into a shared-memory plane with a zero halo of
+//     6, so the x and y neighbours are unconditional loads (the window
+//     truncation falls out of the halo); the pair shares its x-arm loads (16
+//     bytes each) and the RY rows their y-arm loads;
 //   * the 2 FDN + 1 planes of a column's stencil: the centre and the FDN
 //     planes ahead in registers, the FDN planes behind in the thread's own
 //     slots of a shared ring (no barrier: no other thread reads them);
 //   * the shared planes rotate through three buffers under a split barrier:
-//     a thread writes plane z + 1 and arrives on an mbarrier before it works
+//     a warp writes plane z + 1 and arrives on an mbarrier before it works
 //     on plane z, and waits for that phase (bounded) only afterwards, so
 //     warps drift by up to a plane instead of meeting at every plane;
 //   * the nonlocal term reads the layered projector fields (sqb_internal.cuh):
@@ -49,7 +50,6 @@ namespace sqb {
 namespace sweep {
 
 constexpr int KL = LAYERS;
-constexpr int RY_DEFAULT = 2;  // window rows per thread (3 for fields with three projectors per slot)
 
 // Sweep kinds: the Lanczos start vector's projections only; a Lanczos step;
 // a Chebyshev step; a Chebyshev step that also accumulates the density-matrix
@@ -57,7 +57,7 @@ constexpr int RY_DEFAULT = 2;  // window rows per thread (3 for fields with thre
 enum : int { SK_ONES = 0, SK_LZF = 1, SK_CH = 2, SK_FD = 3 };
 
 struct Shared {
-  unsigned long long pbar;  // plane barrier of the sweeps (mbarrier, one arrival per thread and plane)
+  unsigned long long pbar;  // plane barrier of the sweeps (mbarrier, one arrival per warp and plane)
   unsigned pbar_phase;      // its phases completed so far
   int wabort;               // a plane wait ran out of time: later waits are skipped
   int node, qidx, gi, gj, gk;
@@ -70,6 +70,8 @@ struct Shared {
   double scal2[3];
   double aa[MAXL];
   double bb[MAXL];
+  double b2[MAXL];  // bb^2
+  double ger[2];    // Gershgorin interval of the rows whose both neighbours are known
   double eig[2], eprev[2];
   double wdel[2];   // last changes of the extremes (warm start of the next multisection)
   int warm;         // eig holds the extremes of the previous, one row smaller tridiagonal
@@ -92,41 +94,47 @@ struct Shared {
   double pw_prev[MAXP];  // Lanczos: chi^T W_m-1
 };
 
-__host__ __device__ constexpr int plane_pitch(int n) { return n + 2 * FDN; }
+// Thread tile: a pair of adjacent window columns (one 16-byte shared or global
+// access in FP64) and RY adjacent rows.  The pairs start at even columns of the
+// extended grid, so a window that starts at an odd column is shifted by one
+// (sh = gi & 1): window column x sits at pair column x + sh of 0 .. n, and one
+// pad column per row (x = -1 or x = n) carries zeros.  Window vectors, plane
+// buffers and flush slots use this pair layout, rows of pair_cols(n) values.
+__host__ __device__ constexpr int pair_cols(int n) { return n + 1; }  // n is odd
+__host__ __device__ constexpr size_t vec_points(int n) { return (size_t)n * n * pair_cols(n); }
+// Plane buffer pitch: the row with its halo, even (16-byte rows), and where
+// that is possible = the pairs per row modulo 8, so that eight lanes that run
+// over a row's end into the next row of tiles still touch distinct banks.
+__host__ __device__ constexpr int plane_pitch(int n) {
+  const int hx = pair_cols(n) / 2, p = pair_cols(n) + 2 * FDN;
+  return hx % 2 ? p : p + ((hx - p) % 8 + 8) % 8;
+}
+__host__ __device__ constexpr int plane_rows(int n, int ry) { return n + 2 * FDN + ry - 1; }
 // Halo'd planes of the stencil input: plane z lives in buffer z mod NPLANE.
 // Three buffers let a thread write plane z + 1 before it works on plane z
 // while the slowest thread may still read plane z - 1 (see sweep).
 constexpr int NPLANE = 3;
-// NPLANE halo'd planes, plus ry - 1 rows of slack: the shared y-arm loads of
-// a row group whose last rows lie beyond the window read up to ry - 1 rows
-// past the plane (into values that are not used)
 __host__ __device__ inline size_t planes_bytes(int n, int ry) {
-  const int P = plane_pitch(n);
-  return ((size_t)(NPLANE * P * P + (ry - 1) * P + 8) * sizeof(double) + 127) & ~size_t(127);
+  return ((size_t)NPLANE * plane_pitch(n) * plane_rows(n, ry) * sizeof(double) + 127) & ~size_t(127);
 }
 // Lanczos sweeps of the one-projector fields also accumulate the dot products
 // of their input (the exact chi^T W_m, see lanczos), flushed into a second
 // set of the flush buffer.  The buffer (per CTA, after the three window
-// vectors in the scratch) holds [set][layer][projector][plane][column].
+// vectors in the scratch) holds [set][layer][projector][plane][row][pair column].
 __host__ __device__ constexpr bool input_dots(int pm) { return pm == 1; }
 __host__ __device__ inline size_t flush_doubles(int n, int pm) {
-  return (size_t)(input_dots(pm) ? 2 : 1) * KL * pm * n * n * n;
+  return (size_t)(input_dots(pm) ? 2 : 1) * KL * pm * vec_points(n);
 }
 __host__ __device__ inline size_t shared_fixed() { return (sizeof(Shared) + 127) & ~size_t(127); }
-// The threads' rings of the FDN planes behind (RSLOT slots, sized for FP64).
-constexpr int RSLOT = 8;
-__host__ __device__ constexpr bool uses_ring(int pm) { return pm >= 1; }
-__host__ __device__ inline size_t ring_bytes(int nsweep, int pm, int ry) {
-  return uses_ring(pm) ? (((size_t)RSLOT * ry * nsweep * sizeof(double) + 127) & ~size_t(127)) : 0;
-}
-// Lanczos sweeps' input-dot partials, one slot per (layer, row, thread): the
-// owning thread accumulates, flushes and clears its own slots.
-__host__ __device__ inline size_t accw_bytes(int nsweep, int pm, int ry) {
-  return input_dots(pm) ? (((size_t)KL * ry * nsweep * sizeof(double) + 127) & ~size_t(127)) : 0;
+// The threads' rings of the FDN planes behind: a plane's slot is free once the
+// step FDN planes later has read it, which is the step that refills it.  The
+// slots are a compile-time stride (the tile's launch bound) apart.
+constexpr int RSLOT = FDN;
+__host__ __device__ constexpr size_t ring_bytes(int maxt, int ry) {
+  return (size_t)RSLOT * ry * maxt * 2 * sizeof(double);
 }
 __host__ __device__ inline int sweep_threads_of(int n, int ry) {
-  const int groups = (n + ry - 1) / ry;
-  const int t = n <= 32 ? 32 * groups : ((n * groups + 31) / 32) * 32;  // see the thread mapping in sweep
+  const int t = (pair_cols(n) / 2 * ((n + ry - 1) / ry) + 31) / 32 * 32;
   return t < 64 ? 64 : t;  // two warps at least: the multisection's two extremes
 }
 
@@ -141,9 +149,9 @@ __device__ __forceinline__ void bar_sweep(int nthreads) {
   asm volatile("bar.sync 1, %0;\n" ::"r"(nthreads) : "memory");
 }
 
-// The plane barrier: an mbarrier in shared memory that every thread of the
-// block arrives on once per plane (release: its plane writes are visible to
-// the threads whose wait on that phase returns, acquire).
+// The plane barrier: an mbarrier in shared memory that every warp of the block
+// arrives on once per plane, after a __syncwarp (release: the warp's plane
+// writes are visible to the threads whose wait on that phase returns, acquire).
 __device__ __forceinline__ unsigned pbar_addr(const unsigned long long *bar) {
   return (unsigned)__cvta_generic_to_shared(bar);
 }
@@ -167,18 +175,18 @@ __device__ __forceinline__ unsigned long long gtimer_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// Every thread of the block arrives once per plane, so a phase completes in
-// microseconds; a wait that outlasts PBAR_WAIT_NS means a thread stopped
+// Every warp of the block arrives once per plane, so a phase completes in
+// microseconds; a wait that outlasts PBAR_WAIT_NS means a warp stopped
 // arriving: the wait sets the status bit and the block's abort flag, after
 // which no plane wait blocks (the step's results are then void and the call
 // returns an error).
 constexpr unsigned long long PBAR_WAIT_NS = 2000000000ull;
 __device__ __forceinline__ void pbar_wait(Shared &S, int *status, unsigned phase) {
-  if (*(volatile int *)&S.wabort) return;
   const unsigned parity = phase & 1u;
   if (pbar_try_wait(&S.pbar, parity)) return;
   const unsigned long long t0 = gtimer_ns();
   while (!pbar_try_wait(&S.pbar, parity)) {
+    if (*(volatile int *)&S.wabort) return;
     if (gtimer_ns() - t0 > PBAR_WAIT_NS) {
       *(volatile int *)&S.wabort = 1;
       atomicOr(status, ST_WAIT_LIMIT);
@@ -189,7 +197,7 @@ __device__ __forceinline__ void pbar_wait(Shared &S, int *status, unsigned phase
 // Set up the plane barrier at the start of a kernel (before any sweep).
 __device__ __forceinline__ void pbar_setup(Shared &S) {
   if (threadIdx.x == 0) {
-    pbar_init(&S.pbar, blockDim.x);
+    pbar_init(&S.pbar, blockDim.x / 32);
     S.pbar_phase = 0u;
     S.wabort = 0;
   }
@@ -205,10 +213,7 @@ struct IO {
   T *wout = nullptr;       // LZF: where the formed W_m is stored
   double s1 = 1.0;         // LZF: W_m = s1 (Y - ca W1) - cb W2
   double ca = 0.0, cb = 0.0;  // LZF: a, b s; CH: chi, zee
-  double sin = 1.0;        // LZF konst 1: scale of the start vector
-  double chk = 0.0;        // start vector 1 + chk (-1)^(x+y+z)
-  int konst = 0;           // input generated: 1 the (scaled) start vector, 2 the node's unit vector e_c
-  int p1_delta = 0;        // CH: t_k-1 is e_c
+  double chk = 0.0;        // ONES: start vector 1 + chk (-1)^(x+y+z)
   int first = 0;           // CH: t_1 = (H t_0 - chi t_0) / zee (no t_k-1 term)
   int dbl = 0;             // CH: accumulate <t_k+1, t_k+1> and <t_k+1, t_k> (doubling)
   double *dacc = nullptr;  // FD: density-matrix column, FP64
@@ -216,7 +221,8 @@ struct IO {
 };
 
 // Lanczos start vector at window index g: 1 + chk (-1)^(x+y+z); the window
-// edge n is odd, so x + y + z and g = (z n + y) n + x have the same parity.
+// edge n is odd, so x + y + z and g = (z n + y) n + x have the same parity, and
+// any g of that parity will do.
 __device__ __forceinline__ double start_val(double chk, int g) { return 1.0 + chk * (1.0 - 2.0 * (double)(g & 1)); }
 
 __device__ __forceinline__ unsigned lay_of(unsigned long long w, int k) {
@@ -225,224 +231,282 @@ __device__ __forceinline__ unsigned lay_of(unsigned long long w, int k) {
 
 template <typename T>
 __device__ __forceinline__ T *slot(const SweepArgs &a, int k) {
-  const size_t nw = (size_t)a.n * a.n * a.n;
-  return reinterpret_cast<T *>(a.scratch + blockIdx.x * a.scratch_stride + (size_t)k * nw * sizeof(double));
+  return reinterpret_cast<T *>(a.scratch + blockIdx.x * a.scratch_stride + (size_t)k * vec_points(a.n) * sizeof(double));
 }
 
-// Sum of one projector instance's flushed column partials over its box's
-// columns, at the slots of its ball's last window plane (one warp, fixed
-// order), into p_nxt; with IND also the input dots of the second set, into
-// p_in.  The loads of a pass are independent, so they overlap.
+// Sums of the flushed column partials of every projector instance over its
+// box's columns, at the slots of its ball's last window plane, into p_nxt;
+// with IND also the input dots of the second set, into p_in.  Eight lanes per
+// instance in a fixed order, four instances per warp at a time, eight loads
+// in flight per lane: the loads' latency is what this costs.
 template <int PM, bool IND>
-__device__ __forceinline__ void reduce_instance(const SweepArgs &a, Shared &S, const double *fb, int p, int lane) {
-  const int e = S.pi_e[p], q = p - S.e_pb[e], k = S.e_k[e];
-  const int n = a.n, n2 = n * n;
-  const int x0 = S.e_x0[e], y0 = S.e_y0[e];
-  const int bx = S.e_x1[e] - x0 + 1, by = S.e_y1[e] - y0 + 1, cnt = bx * by;
-  const int base = ((k * PM + q) * n + S.e_z1[e]) * n2 + y0 * n + x0, set = KL * PM * n * n2;
-  const double *f = fb + base;
-  const double *fw = f + set;
-  (void)set;
-  double s = 0.0, sw = 0.0;
-#pragma unroll 4
-  for (int i = lane; i < cnt; i += 32) {
-    const int yy = i / bx, xx = i - yy * bx;
-    const int o = SQB_IDX(base + yy * n + xx, set, a.status) - base;
-    s += f[o];
-    if constexpr (IND) sw += fw[o];
-  }
-  s = warp_sum(s);
-  if constexpr (IND) sw = warp_sum(sw);
-  if (lane == 0) {
-    S.p_nxt[p] = s;
-    if constexpr (IND) S.p_in[p] = sw;
+__device__ __forceinline__ void reduce_instances(const SweepArgs &a, Shared &S, const double *fb, int warp, int nwarp,
+                                                 int lane) {
+  const int n = a.n, NP = pair_cols(n), plane = n * NP, set = KL * PM * n * plane;
+  const int sh = S.gi & 1, sub = lane & 7;
+  for (int p0 = warp * 4; p0 < S.n_pi; p0 += nwarp * 4) {
+    const int p = p0 + (lane >> 3);
+    double s = 0.0, sw = 0.0;
+    if (p < S.n_pi) {
+      const int e = S.pi_e[p], q = p - S.e_pb[e], k = S.e_k[e];
+      const int x0 = S.e_x0[e], y0 = S.e_y0[e];
+      const int bx = S.e_x1[e] - x0 + 1, cnt = bx * (S.e_y1[e] - y0 + 1);
+      const int base = ((k * PM + q) * n + S.e_z1[e]) * plane + y0 * NP + x0 + sh;
+      // i / bx for i < 43 * 43 by a 2^20 reciprocal: the excess i (inv bx - 2^20) / (bx 2^20) stays below 1 / bx
+      const unsigned inv = ((1u << 20) + bx - 1) / bx;
+      const double *f = fb + base;
+      for (int i0 = sub; i0 < cnt; i0 += 64) {
+        double v[8], w[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const int i = i0 + 8 * t, yy = (int)(((unsigned)i * inv) >> 20);
+          const bool in = i < cnt;
+          const int o = in ? SQB_IDX(base + yy * NP + (i - yy * bx), set, a.status) - base : 0;
+          v[t] = in ? f[o] : 0.0;
+          if constexpr (IND) w[t] = in ? f[o + set] : 0.0;
+        }
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          s += v[t];
+          if constexpr (IND) sw += w[t];
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      if constexpr (IND) sw += __shfl_xor_sync(0xffffffffu, sw, o);
+    }
+    if (sub == 0 && p < S.n_pi) {
+      S.p_nxt[p] = s;
+      if constexpr (IND) S.p_in[p] = sw;
+    }
   }
 }
 
-// One sweep over the window's z-planes (all threads of the block).  The
-// stencil input of a thread's rows: with the ring, the centre and the FDN
-// planes ahead in registers (fut[j][0] the centre, fut[j][s] plane z + s) and
-// the FDN planes behind in the thread's own slots of a shared ring (plane
-// z - s in slot (z - s) mod RSLOT); without it, all 2 FDN + 1 planes in
-// registers (fut[j][FDN + s] plane z + s).
-template <typename T, int PM, int SK, int RY>
+// All plane buffers to zero (the halo; the sweeps write the interior).  Once
+// per kernel, and where the buffers change between FP32 and FP64 values.
+static __device__ void zero_planes(const SweepArgs &a, unsigned char *dyn, int ry) {
+  __syncthreads();
+  uint4 *p = reinterpret_cast<uint4 *>(dyn);
+  for (int i = threadIdx.x; i < (int)(planes_bytes(a.n, ry) / 16); i += blockDim.x) p[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+}
+
+template <typename T>
+struct PairOf;
+template <>
+struct PairOf<double> {
+  using type = double2;
+};
+template <>
+struct PairOf<float> {
+  using type = float2;
+};
+
+// One sweep over the window's z-planes (all threads of the block).  A
+// thread's stencil input along z: the centre and the FDN planes ahead in
+// registers (fut[j][0] the centre, fut[j][s] plane z + s) and the FDN planes
+// behind in the thread's own slots of a shared ring.
+//
+// What bounds it is latency and instruction issue (B200, 31^3 windows, force
+// sweeps: 52% of issue slots, 65% inside the plane loop; 334 thread
+// instructions per point, 118 of them integer and 57 FP64), not FP64 (13% of
+// the pipe) and not memory (57 bytes per point, from L2).  A pair of columns
+// per thread takes its x-arm values in 3 16-byte loads per point where a single
+// column takes 12 8-byte ones.  The streamed operands bypass L1 (__ldcg,
+// __stcg), which the shared memory leaves small, so that it keeps the spilled
+// registers: with them in it 60% of the spill loads went to L2.
+template <typename T, int PM, int SK, int RY, int NT>
 __device__ __forceinline__ void sweep(const SweepArgs &a, Shared &S, unsigned char *dyn, const IO<T> &io,
                                       double &acc0, double &acc1) {
+  using T2 = typename PairOf<T>::type;
   constexpr bool STENCIL = SK != SK_ONES;
   constexpr bool CHEB = SK == SK_CH || SK == SK_FD;
-  constexpr bool RING = uses_ring(PM);
-  constexpr int F = RING ? FDN + 1 : 2 * FDN + 1;  // planes held in registers
-  constexpr int C = RING ? 0 : FDN;                // register index of the centre
-  constexpr bool CHR = PM == 1;  // projector values kept in registers from one plane to the next
+  constexpr int F = FDN + 1;       // planes held in registers
+  constexpr bool CHR = PM == 1;    // projector values kept in registers from one plane to the next
   constexpr bool IND = SK == SK_LZF && input_dots(PM);  // dot products of the input too
-  const int n = a.n, n2 = n * n, P = plane_pitch(n), P2 = P * P;
+  const int n = a.n, NP = pair_cols(n), HX = NP >> 1, P = plane_pitch(n), PB = P * plane_rows(n, RY);
   const int tid = threadIdx.x, NS = a.nsweep, lane = tid & 31, warp = tid >> 5, nwarp = NS >> 5;
-  // thread -> (column x, row group): windows up to 32 wide give each row
-  // group a warp of its own (lane = column), so no warp straddles two row
-  // groups and its shared-plane loads are one contiguous run (no bank
-  // conflicts); wider windows pack the columns densely
-  const int nrow = (n + RY - 1) / RY;
-  const bool lanes = n <= 32;
-  const int tx = lanes ? (tid & 31) : tid % n, tg = lanes ? (tid >> 5) : tid / n;
-  const bool tv = tx < n && tg < nrow;
-  const int x = tv ? tx : 0, yb = tv ? tg * RY : 0;
-  const int nl = a.nloc, gc = (nl * n + nl) * n + nl;  // window index of the centre
+  const int tg = tid / HX, px = tid - tg * HX;
+  const bool tv = tg * RY < n;
+  const int sh = S.gi & 1;
+  const int xx = 2 * px, yb = tv ? tg * RY : 0;  // pair column, first row
+  const bool cv0 = !(sh && px == 0), cv1 = sh || px != HX - 1;  // columns inside the window
+  const int nl = a.nloc;
   const int EP = a.ex * a.ey, EV = (int)a.evol;  // the extended grid fits 32-bit indices
+  const int VP = n * NP, NW = n * VP;            // values per plane and per window vector
   const unsigned dummy = (unsigned)a.n_gproj;
   const unsigned long long empty = 0x0001000100010001ull * (unsigned long long)dummy;  // no ball in any layer
   T *sm = reinterpret_cast<T *>(dyn);
-  T *ring = reinterpret_cast<T *>(dyn + planes_bytes(n, RY));
-  double *accw = reinterpret_cast<double *>(dyn + planes_bytes(n, RY) + ring_bytes(NS, PM, RY));
-  const double *pcur =
-      reinterpret_cast<const double *>(dyn + planes_bytes(n, RY) + ring_bytes(NS, PM, RY) + accw_bytes(NS, PM, RY));
-  double *fb = slot<double>(a, 3);                // flush buffer: [set][layer][projector][plane][column]
-  double *fbw = fb + (size_t)KL * PM * n * n2;  // IND: the input's set
-  const double *veff = a.veff64;
-  const unsigned long long *lid = a.lay_id;
-  const double *lchi = a.lay_chi;
-  const int NW = n * n2;                     // window points (vector length)
-  int *const st = a.status;                  // (bounds-check build)
-  (void)NW;
+  T2 *ring = reinterpret_cast<T2 *>(dyn + planes_bytes(n, RY)) + tid;
+  constexpr int RS = RY * NT;  // pairs per ring slot
+  const double *pcur = reinterpret_cast<const double *>(dyn + planes_bytes(n, RY) + ring_bytes(NT, RY));
+  double *fb = slot<double>(a, 3);  // flush buffer: [set][layer][projector][plane][row][pair column]
+  const int fset = KL * PM * NW;
+  int *const st = a.status;  // (bounds-check build)
   (void)st;
+  (void)EV;
 
-  // zero the halo of the planes (the interior is written every plane)
-  for (int i = tid; i < NPLANE * P2; i += NS) {
-    const int r = (i % P2) / P, c = i % P;
-    if (r < FDN || r >= n + FDN || c < FDN || c >= n + FDN) sm[i] = T(0);
-  }
-
-  int y[RY], col[RY];
   bool ok[RY];
-  int xb[RY];
 #pragma unroll
-  for (int j = 0; j < RY; j++) {
-    y[j] = yb + j;
-    ok[j] = tv && y[j] < n;
-    col[j] = ok[j] ? y[j] * n + x : 0;
-    xb[j] = (S.gk * a.ey + (S.gj + (ok[j] ? y[j] : 0))) * a.ex + S.gi + x;
-  }
-  // ring slot of (row j, plane zz): ring[((zz mod RSLOT) * RY + j) * NS + tid]
-  auto rslot = [&](int j, int zz) -> T & { return ring[(((zz + RSLOT) & (RSLOT - 1)) * RY + j) * NS + tid]; };
+  for (int j = 0; j < RY; j++) ok[j] = tv && yb + j < n;
+  const int g0 = yb * NP + xx;                                                       // window vectors, plane 0
+  const int X0 = (S.gk * a.ey + S.gj + yb) * a.ex + S.gi - sh + xx;                  // fields, plane 0
+  // the thread that owns the window centre: row cj of its tile, column cc of its pair
+  const bool ctr = tv && xx == ((nl + sh) & ~1) && yb <= nl && nl < yb + RY;
+  const int cj = nl - yb, cc = (nl + sh) & 1;
+  const unsigned par0 = (unsigned)(xx - sh + yb) & 1u;  // parity of x + y of the tile's first point
 
   // the stencil input of row j at plane zz (LZF: formed from the loaded operands)
-  T fut[RY][F];
-  T pf[RY], r1[RY], r2[RY];
+  T2 fut[RY][F];
+  T2 pf[RY], r1[RY], r2[RY];
   auto load_ops = [&](int j, int zz) {
-    if (!ok[j] || zz >= n || io.konst) return;
-    const int g = SQB_IDX(zz * n2 + col[j], NW, st);
-    pf[j] = io.vin[g];
+    if (!ok[j] || zz >= n) return;
+    const int g = SQB_IDX(g0 + zz * VP + j * NP, NW - 1, st);
+    pf[j] = __ldcg(reinterpret_cast<const T2 *>(io.vin + g));
     if constexpr (SK == SK_LZF) {
-      r1[j] = io.p1[g];
-      r2[j] = io.p2[g];
+      r1[j] = __ldcg(reinterpret_cast<const T2 *>(io.p1 + g));
+      r2[j] = __ldcg(reinterpret_cast<const T2 *>(io.p2 + g));
     }
   };
-  auto next_in = [&](int j, int zz) -> T {
-    if (!ok[j] || zz >= n) return T(0);
-    const int g = zz * n2 + col[j];
-    T v;
-    if (io.konst == 1) v = (T)(io.sin * start_val(io.chk, g));
-    else if (io.konst == 2) v = (T)(g == gc ? 1.0 : 0.0);
-    else if constexpr (SK == SK_LZF) v = (T)(io.s1 * ((double)pf[j] - io.ca * (double)r1[j]) - io.cb * (double)r2[j]);
-    else v = pf[j];
-    if constexpr (SK == SK_LZF) io.wout[SQB_IDX(g, NW, st)] = v;
+  auto next_in = [&](int j, int zz) -> T2 {
+    T2 v;
+    v.x = v.y = T(0);
+    if (!ok[j] || zz >= n) return v;
+    if constexpr (SK == SK_LZF) {
+      v.x = (T)(io.s1 * ((double)pf[j].x - io.ca * (double)r1[j].x) - io.cb * (double)r2[j].x);
+      v.y = (T)(io.s1 * ((double)pf[j].y - io.ca * (double)r1[j].y) - io.cb * (double)r2[j].y);
+    } else {
+      v = pf[j];
+    }
+    if constexpr (SK == SK_LZF)
+      __stcg(reinterpret_cast<T2 *>(io.wout + SQB_IDX(g0 + zz * VP + j * NP, NW - 1, st)), v);
     return v;
   };
 
   // per-plane point data, loaded one plane ahead
-  double ve[RY];
-  T q1[RY];
-  double dq[RY];  // FD: D at the point, loaded one plane ahead
-  unsigned long long idc[RY], idn[RY];
-  double chc[RY][KL][PM];
-  double acd[RY][KL][PM];
-  // IND: the input's partial of (layer k, row j) lives in accw[(k RY + j) NS + tid]
-  auto load_ids = [&](int j, int zz) -> unsigned long long {
-    return (ok[j] && zz < n) ? __ldg(lid + SQB_IDX(xb[j] + zz * EP, EV, st)) : empty;
+  double2 ve[RY];
+  T2 q1[RY];
+  double2 dq[RY];  // FD: D at the point
+  unsigned long long idc[RY][2] = {}, idn[RY][2] = {};
+  double2 chc[RY][KL];       // CHR: projector values
+  double2 acd[RY][KL][PM];   // dot products with the output, per column and current ball
+  double2 acw[RY][KL];       // IND: with the input
+  auto load_ids = [&](int j, int zz) {
+    ulonglong2 v = make_ulonglong2(empty, empty);
+    if (ok[j] && zz < n)
+      v = __ldcg(reinterpret_cast<const ulonglong2 *>(a.lay_id + SQB_IDX(X0 + zz * EP + j * a.ex, EV - 1, st)));
+    idn[j][0] = v.x;
+    idn[j][1] = v.y;
+  };
+  auto chi_ld = [&](int j, int kq, int k, int X) -> double2 {
+    double2 v = make_double2(0.0, 0.0);
+    if (lay_of(idc[j][0], k) != dummy || lay_of(idc[j][1], k) != dummy)
+      v = CHR ? __ldcg(reinterpret_cast<const double2 *>(a.lay_chi + (size_t)kq * EV + X))
+              : __ldg(reinterpret_cast<const double2 *>(a.lay_chi + (size_t)kq * EV + X));
+    return v;
   };
   auto load_point = [&](int j, int zz) {
     if (!ok[j] || zz >= n) return;
-    const int X = SQB_IDX(xb[j] + zz * EP, EV, st);
-    if constexpr (STENCIL) ve[j] = __ldg(veff + X);
+    const int X = SQB_IDX(X0 + zz * EP + j * a.ex, EV - 1, st);
+    if constexpr (STENCIL) ve[j] = __ldcg(reinterpret_cast<const double2 *>(a.veff64 + X));
     if constexpr (CHEB) {
-      if (!io.first)
-        q1[j] = io.p1_delta ? (T)(zz * n2 + col[j] == gc ? 1.0 : 0.0) : io.p1[SQB_IDX(zz * n2 + col[j], NW, st)];
+      if (!io.first) {
+        q1[j] = __ldcg(reinterpret_cast<const T2 *>(io.p1 + SQB_IDX(g0 + zz * VP + j * NP, NW - 1, st)));
+      }
     }
-    if constexpr (SK == SK_FD) dq[j] = io.first ? 0.0 : io.dacc[SQB_IDX(zz * n2 + col[j], NW, st)];
+    if constexpr (SK == SK_FD) {
+      if (!io.first) dq[j] = __ldcg(reinterpret_cast<const double2 *>(io.dacc + SQB_IDX(g0 + zz * VP + j * NP, NW - 1, st)));
+    }
     if constexpr (CHR) {
 #pragma unroll
-      for (int k = 0; k < KL; k++)
-        chc[j][k][0] = lay_of(idc[j], k) != dummy ? __ldg(lchi + k * EV + X) : 0.0;
+      for (int k = 0; k < KL; k++) chc[j][k] = chi_ld(j, k, k, X);
     }
-  };
-  auto chi_at = [&](int j, int k, int q, int X) -> double {
-    if constexpr (CHR) return chc[j][k][0];
-    else return lay_of(idc[j], k) != dummy ? __ldg(lchi + (k * PM + q) * EV + X) : 0.0;
   };
 
 #pragma unroll
   for (int j = 0; j < RY; j++) {
-    ve[j] = 0.0;
-    q1[j] = T(0);
-    dq[j] = 0.0;
+    ve[j] = dq[j] = make_double2(0.0, 0.0);
+    q1[j].x = q1[j].y = T(0);
+    load_ids(j, 0);
+#pragma unroll
+    for (int i = 0; i < 2; i++) idc[j][i] = idn[j][i];
 #pragma unroll
     for (int k = 0; k < KL; k++) {
-      if constexpr (IND) accw[(k * RY + j) * NS + tid] = 0.0;
+      acw[j][k] = chc[j][k] = make_double2(0.0, 0.0);
 #pragma unroll
-      for (int q = 0; q < PM; q++) acd[j][k][q] = chc[j][k][q] = 0.0;
+      for (int q = 0; q < PM; q++) acd[j][k][q] = make_double2(0.0, 0.0);
     }
-    idc[j] = load_ids(j, 0);
-    idn[j] = load_ids(j, 1);
+    load_ids(j, 1);
     if constexpr (STENCIL) {
       // planes behind the window are zero; planes 0..FDN enter it
-      if constexpr (RING) {
+      T2 zero;
+      zero.x = zero.y = T(0);
 #pragma unroll
-        for (int s = 1; s <= FDN; s++) rslot(j, -s) = T(0);
-      } else {
-#pragma unroll
-        for (int s = 0; s < FDN; s++) fut[j][s] = T(0);
-      }
+      for (int s = 0; s < RSLOT; s++) ring[s * RS + j * NT] = zero;
+      T2 pp[FDN + 1], pr1[FDN + 1], pr2[FDN + 1];  // (all loads in flight before the first stored plane)
 #pragma unroll
       for (int s = 0; s <= FDN; s++) {
         load_ops(j, s);
-        fut[j][C + s] = next_in(j, s);
+        pp[s] = pf[j];
+        if constexpr (SK == SK_LZF) {
+          pr1[s] = r1[j];
+          pr2[s] = r2[j];
+        }
+      }
+#pragma unroll
+      for (int s = 0; s <= FDN; s++) {
+        pf[j] = pp[s];
+        if constexpr (SK == SK_LZF) {
+          r1[j] = pr1[s];
+          r2[j] = pr2[s];
+        }
+        fut[j][s] = next_in(j, s);
       }
       load_ops(j, FDN + 1);
     }
     load_point(j, 0);
   }
   const double c0 = 3.0 * a.coeff_lap[0];
-  const double rcb = CHEB ? 1.0 / io.cb : 0.0;
+  const double rcb = CHEB ? (io.first ? 1.0 : 2.0) / io.cb : 0.0;  // (2/zee is exactly twice 1/zee)
   const double cdh = io.cd / a.h3, ceh = io.ce / a.h3;
+  unsigned big = 0u;  // largest magnitude word of the outputs (non-finite check)
 
   // Planes through the shared buffers with a split barrier: in step z a
   // thread first writes its centre values of plane z + 1 (buffer (z+1) mod 3)
-  // and arrives, then works on plane z, and only then waits until every
-  // thread has written plane z + 1.  A thread in step z has seen every thread
+  // and its warp arrives, then works on plane z, and only then waits until
+  // every warp has written plane z + 1.  A warp in step z has seen every warp
   // arrive in step z - 1, so the slowest is at worst in step z - 1, reading
   // buffer (z-1) mod 3: one buffer apart from the one written.  Warps drift
   // by up to a plane instead of meeting at every plane.
-  const int sofs = (yb + FDN) * P + x + FDN;  // the thread's first row in a plane buffer
+  const int sofs = (yb + FDN) * P + xx + FDN;  // the thread's first row in a plane buffer
   if constexpr (STENCIL) {
+    if (tv) {
 #pragma unroll
-    for (int j = 0; j < RY; j++)
-      if (ok[j]) sm[sofs + j * P] = fut[j][C];
+      for (int j = 0; j < RY; j++) *reinterpret_cast<T2 *>(sm + sofs + j * P) = fut[j][0];
+    }
   }
-  bar_sweep(NS);  // halo and plane 0 written; the previous sweep's phases are counted
+  bar_sweep(NS);  // plane 0 written; the previous sweep's phases are counted
   const unsigned ph0 = S.pbar_phase;
   int bz = 0;  // buffer of plane z
+  int rz = 0;  // ring slot of plane z (and of plane z - RSLOT)
   for (int z = 0; z < n; z++) {
-    T *smz = sm + bz * P2;
+    const T *smz = sm + bz * PB;
     const int bn = bz == NPLANE - 1 ? 0 : bz + 1;
     if constexpr (STENCIL) {
       if (z + 1 < n) {
+        if (tv) {
 #pragma unroll
-        for (int j = 0; j < RY; j++)
-          if (ok[j]) sm[bn * P2 + sofs + j * P] = fut[j][C + 1];
-        pbar_arrive(&S.pbar);
+          for (int j = 0; j < RY; j++) *reinterpret_cast<T2 *>(sm + bn * PB + sofs + j * P) = fut[j][1];
+        }
+        __syncwarp();
+        if (lane == 0) pbar_arrive(&S.pbar);
       }
     }
     if (tv) {
-      double hv[RY], v[RY];
+      double2 hv[RY], v[RY];
       if constexpr (STENCIL) {
         // arm k of each point sums (x-k) + (x+k) + (y-k) + (y+k) + (z-k) + (z+k)
         // in that order before the coefficient, as HsubTimesVec does
@@ -450,113 +514,154 @@ __device__ __forceinline__ void sweep(const SweepArgs &a, Shared &S, unsigned ch
         // y-arm loads: arm k loads rows y0-k (ym[k]) and y0+RY-1+k (yp[k]); row
         // j's y0+j-k is the centre of row j-k when j >= k, else ym[k-j], and
         // its y0+j+k the centre of row j+k when j+k < RY, else yp[j+k-RY+1].
-        const T *cp0 = smz + (yb + FDN) * P + x + FDN;
-        double temp[RY];
+        const T *cp = smz + sofs;
+        double2 temp[RY];
+        T2 xl[RY][FDN / 2 + 1], xr[RY][FDN / 2 + 1];  // pairs at -2s and +2s of the row
+        T2 ym[FDN + 1], yp[FDN + 1];
 #pragma unroll
-        for (int j = 0; j < RY; j++) temp[j] = (double)fut[j][C] * c0;
-        if constexpr (RY == 2) {
-          // the same, with the loads of the previous arm carried in two registers
-          const T *c1p = cp0 + P;
-          T prev_m = fut[0][C], prev_p = fut[1][C];
+        for (int j = 0; j < RY; j++) {
+          temp[j].x = (double)fut[j][0].x * c0;
+          temp[j].y = (double)fut[j][0].y * c0;
+          xl[j][0] = xr[j][0] = fut[j][0];
+        }
 #pragma unroll
-          for (int k = 1; k <= FDN; k++) {
-            const T ym = cp0[-k * P], yp = c1p[k * P];
-            const T zm0 = RING ? rslot(0, z - k) : fut[0][C - k], zm1 = RING ? rslot(1, z - k) : fut[1][C - k];
-            const T s0 = cp0[-k] + cp0[k] + ym + prev_p + zm0 + fut[0][C + k];
-            const T s1 = c1p[-k] + c1p[k] + prev_m + yp + zm1 + fut[1][C + k];
-            temp[0] += (double)s0 * a.coeff_lap[k];
-            temp[1] += (double)s1 * a.coeff_lap[k];
-            prev_m = ym;
-            prev_p = yp;
-          }
-        } else {
-          T ym[FDN + 1], yp[FDN + 1];
+        for (int k = 1; k <= FDN; k++) {
+          ym[k] = *reinterpret_cast<const T2 *>(cp - k * P);
+          yp[k] = *reinterpret_cast<const T2 *>(cp + (RY - 1 + k) * P);
+          const T2 *rb = ring + (rz < k ? rz + RSLOT - k : rz - k) * RS;  // plane z - k
 #pragma unroll
-          for (int k = 1; k <= FDN; k++) {
-            ym[k] = cp0[-k * P];
-            yp[k] = cp0[(RY - 1 + k) * P];
-#pragma unroll
-            for (int j = 0; j < RY; j++) {
-              const T *cj = cp0 + j * P;
-              const T ylo = j >= k ? fut[j - k][C] : ym[k - j];
-              const T yhi = j + k < RY ? fut[j + k][C] : yp[j + k - RY + 1];
-              const T zm = RING ? rslot(j, z - k) : fut[j][C - k];
-              const T sj = cj[-k] + cj[k] + ylo + yhi + zm + fut[j][C + k];
-              temp[j] += (double)sj * a.coeff_lap[k];
+          for (int j = 0; j < RY; j++) {
+            if (k & 1) {  // arms k and k + 1 of the pair reach the pairs at -(k + 1) and k + 1
+              xl[j][(k + 1) / 2] = *reinterpret_cast<const T2 *>(cp + j * P - (k + 1));
+              xr[j][(k + 1) / 2] = *reinterpret_cast<const T2 *>(cp + j * P + (k + 1));
             }
+            // x - k, x + k of the pair's columns
+            const T m0 = (k & 1) ? xl[j][(k + 1) / 2].y : xl[j][k / 2].x;
+            const T p0 = (k & 1) ? xr[j][(k - 1) / 2].y : xr[j][k / 2].x;
+            const T m1 = (k & 1) ? xl[j][(k - 1) / 2].x : xl[j][k / 2].y;
+            const T p1 = (k & 1) ? xr[j][(k + 1) / 2].x : xr[j][k / 2].y;
+            const T2 ylo = j >= k ? fut[j >= k ? j - k : 0][0] : ym[j >= k ? 1 : k - j];
+            const T2 yhi = j + k < RY ? fut[j + k < RY ? j + k : 0][0] : yp[j + k < RY ? 1 : j + k - RY + 1];
+            const T2 zm = rb[j * NT];
+            const T s0 = m0 + p0 + ylo.x + yhi.x + zm.x + fut[j][k].x;
+            const T s1 = m1 + p1 + ylo.y + yhi.y + zm.y + fut[j][k].y;
+            temp[j].x += (double)s0 * a.coeff_lap[k];
+            temp[j].y += (double)s1 * a.coeff_lap[k];
           }
         }
 #pragma unroll
         for (int j = 0; j < RY; j++) {
-          const int X = xb[j] + z * EP;
-          double vnl = 0.0;
+          const int X = X0 + z * EP + j * a.ex;
+          double2 vnl = make_double2(0.0, 0.0);
 #pragma unroll
           for (int k = 0; k < KL; k++) {
-            const unsigned id = lay_of(idc[j], k);
+            const unsigned i0 = lay_of(idc[j][0], k), i1 = lay_of(idc[j][1], k);
 #pragma unroll
-            for (int q = 0; q < PM; q++) vnl += pcur[SQB_IDX(id + q, a.n_gproj + PM, st)] * chi_at(j, k, q, X);
+            for (int q = 0; q < PM; q++) {
+              double2 ch;
+              if constexpr (CHR) ch = chc[j][k];
+              else ch = ok[j] ? chi_ld(j, k * PM + q, k, X) : make_double2(0.0, 0.0);
+              vnl.x += pcur[SQB_IDX(i0 + q, a.n_gproj + PM, st)] * ch.x;
+              vnl.y += pcur[SQB_IDX(i1 + q, a.n_gproj + PM, st)] * ch.y;
+            }
           }
-          v[j] = (double)fut[j][C];
-          hv[j] = -0.5 * temp[j] + ve[j] * v[j] + vnl;
+          v[j].x = (double)fut[j][0].x;
+          v[j].y = (double)fut[j][0].y;
+          hv[j].x = -0.5 * temp[j].x + ve[j].x * v[j].x + vnl.x;
+          hv[j].y = -0.5 * temp[j].y + ve[j].y * v[j].y + vnl.y;
         }
       }
 #pragma unroll
       for (int j = 0; j < RY; j++) {
         if (!ok[j]) continue;
-        const int g = SQB_IDX(z * n2 + col[j], NW, st);
-        double o;
+        const int g = SQB_IDX(g0 + z * VP + j * NP, NW - 1, st);
+        double2 o;
         if constexpr (SK == SK_ONES) {
-          o = start_val(io.chk, g);
-        } else if constexpr (SK == SK_LZF) {
-          const T ot = (T)hv[j];
-          io.out[g] = ot;
-          acc0 += v[j] * v[j];
-          acc1 += v[j] * hv[j];
-          o = (double)ot;
+          const unsigned par = par0 + j + z;
+          o = make_double2(cv0 ? start_val(io.chk, par) : 0.0, cv1 ? start_val(io.chk, par + 1u) : 0.0);
         } else {
-          // sq.cpp:588, 615 divide by zee; the sweep multiplies by 1/zee
-          // (one rounding apart, no FP64 division per point)
-          double od;
-          if (io.first) od = (hv[j] - io.ca * v[j]) * rcb;
-          else od = (2.0 * (hv[j] - io.ca * v[j])) * rcb - (double)q1[j];
-          const T ot = (T)od;
-          io.out[g] = ot;
-          o = (double)ot;
-          if (io.dbl) {
-            acc0 += o * o;
-            acc1 += o * v[j];
+          T2 ot;
+          if constexpr (SK == SK_LZF) {
+            ot.x = cv0 ? (T)hv[j].x : T(0);
+            ot.y = cv1 ? (T)hv[j].y : T(0);
+            acc0 += v[j].x * v[j].x;
+            acc0 += v[j].y * v[j].y;
+            acc1 += v[j].x * hv[j].x;  // (v is zero in the pad column)
+            acc1 += v[j].y * hv[j].y;
+          } else {
+            // sq.cpp:588, 615 divide by zee; the sweep multiplies by 1/zee
+            // (one rounding apart, no FP64 division per point)
+            double2 od;
+            od.x = (hv[j].x - io.ca * v[j].x) * rcb - (double)q1[j].x;
+            od.y = (hv[j].y - io.ca * v[j].y) * rcb - (double)q1[j].y;
+            ot.x = cv0 ? (T)od.x : T(0);
+            ot.y = cv1 ? (T)od.y : T(0);
           }
-          if constexpr (SK == SK_FD) {  // forces.cpp:414-456 (Ci / h^3 formed once per sweep)
-            if (io.first) io.dacc[g] = (g == gc ? ceh : 0.0) + o * cdh;
-            else io.dacc[g] = dq[j] + o * cdh;
+          __stcg(reinterpret_cast<T2 *>(io.out + g), ot);
+          o.x = (double)ot.x;
+          o.y = (double)ot.y;
+          if constexpr (CHEB) {
+            if (io.dbl) {
+              acc0 += o.x * o.x;
+              acc0 += o.y * o.y;
+              acc1 += o.x * v[j].x;
+              acc1 += o.y * v[j].y;
+            }
+            if constexpr (SK == SK_FD) {  // forces.cpp:414-456 (Ci / h^3 formed once per sweep)
+              double2 dn;
+              if (io.first) dq[j] = make_double2(v[j].x * ceh, v[j].y * ceh);  // (the input is e_c)
+              dn.x = dq[j].x + o.x * cdh;
+              dn.y = dq[j].y + o.y * cdh;
+              __stcg(reinterpret_cast<double2 *>(io.dacc + g), dn);
+            }
           }
+          if (z == nl && ctr && j == cj) S.center_val = cc ? o.y : o.x;
+          big = max(big, max((unsigned)__double2hiint(o.x) & 0x7fffffffu, (unsigned)__double2hiint(o.y) & 0x7fffffffu));
         }
-        if (g == gc) S.center_val = o;
-        if (!isfinite(o)) atomicOr(a.status, ST_NONFINITE);
-        const int X = xb[j] + z * EP;
+        const int X = X0 + z * EP + j * a.ex;
+        (void)X;
 #pragma unroll
         for (int k = 0; k < KL; k++) {
 #pragma unroll
-          for (int q = 0; q < PM; q++) acd[j][k][q] += chi_at(j, k, q, X) * o;
-          if constexpr (IND) {
-            if (lay_of(idc[j], k) != dummy) accw[(k * RY + j) * NS + tid] += chi_at(j, k, 0, X) * v[j];
+          for (int q = 0; q < PM; q++) {
+            double2 ch;
+            if constexpr (CHR) ch = chc[j][k];
+            else ch = chi_ld(j, k * PM + q, k, X);
+            acd[j][k][q].x += ch.x * o.x;
+            acd[j][k][q].y += ch.y * o.y;
+            if constexpr (IND) {
+              acw[j][k].x += ch.x * v[j].x;
+              acw[j][k].y += ch.y * v[j].y;
+            }
           }
         }
-        // a column that leaves a layer's ball after plane z flushes its partial
-        // to the slot of (layer, z, column)
-        const unsigned long long chg = idc[j] ^ idn[j];
-        if (z + 1 < n && chg != 0ull) {
+      }
+      // a column that leaves a layer's ball after plane z flushes its partial
+      // to the slot of (layer, z, column) and takes the next ball's coefficient
+      unsigned long long chg = 0ull;
 #pragma unroll
-          for (int k = 0; k < KL; k++) {
-            if (lay_of(chg, k) == 0u) continue;
-            if (lay_of(idc[j], k) != dummy) {
+      for (int j = 0; j < RY; j++) chg |= (idc[j][0] ^ idn[j][0]) | (idc[j][1] ^ idn[j][1]);
+      if (z + 1 < n && chg != 0ull) {
 #pragma unroll
-              for (int q = 0; q < PM; q++) fb[SQB_IDX(((k * PM + q) * n + z) * n2 + col[j], KL * PM * NW, st)] = acd[j][k][q];
-              if constexpr (IND) fbw[(k * n + z) * n2 + col[j]] = accw[(k * RY + j) * NS + tid];
+        for (int k = 0; k < KL; k++) {
+          if (lay_of(chg, k) == 0u) continue;
+#pragma unroll
+          for (int j = 0; j < RY; j++) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+              const unsigned was = lay_of(idc[j][i], k), now = lay_of(idn[j][i], k);
+              if (was != now) {
+                if (was != dummy) {
+                  const int f = SQB_IDX((k * PM * n + z) * VP + g0 + j * NP + i, fset - (PM - 1) * NW, st);
+#pragma unroll
+                  for (int q = 0; q < PM; q++) fb[f + q * NW] = i ? acd[j][k][q].y : acd[j][k][q].x;
+                  if constexpr (IND) fb[f + fset] = i ? acw[j][k].y : acw[j][k].x;
+                }
+#pragma unroll
+                for (int q = 0; q < PM; q++) (i ? acd[j][k][q].y : acd[j][k][q].x) = 0.0;
+                if constexpr (IND) (i ? acw[j][k].y : acw[j][k].x) = 0.0;
+              }
             }
-#pragma unroll
-            for (int q = 0; q < PM; q++) acd[j][k][q] = 0.0;
-            if constexpr (IND) accw[(k * RY + j) * NS + tid] = 0.0;
           }
         }
       }
@@ -564,11 +669,14 @@ __device__ __forceinline__ void sweep(const SweepArgs &a, Shared &S, unsigned ch
     // advance: ids, point data and the stencil input
 #pragma unroll
     for (int j = 0; j < RY; j++) {
-      idc[j] = idn[j];
-      idn[j] = load_ids(j, z + 2);
+      if (z + 1 < n) {
+        idc[j][0] = idn[j][0];
+        idc[j][1] = idn[j][1];
+      }
+      load_ids(j, z + 2);
       load_point(j, z + 1);
       if constexpr (STENCIL) {
-        if constexpr (RING) rslot(j, z) = fut[j][0];  // plane z moves behind (its slot is free: RSLOT > FDN)
+        ring[rz * RS + j * NT] = fut[j][0];  // plane z moves behind
 #pragma unroll
         for (int s = 0; s < F - 1; s++) fut[j][s] = fut[j][s + 1];
         fut[j][F - 1] = next_in(j, z + FDN + 1);
@@ -579,29 +687,33 @@ __device__ __forceinline__ void sweep(const SweepArgs &a, Shared &S, unsigned ch
       if (z + 1 < n) pbar_wait(S, a.status, ph0 + (unsigned)z);
     }
     bz = bn;
+    rz = rz == RSLOT - 1 ? 0 : rz + 1;
   }
+  if (big >= 0x7ff00000u) atomicOr(a.status, ST_NONFINITE);
   if constexpr (STENCIL) {
     // every thread read ph0 before its first arrival, and thread 0 passed
     // every wait of this sweep
     if (tid == 0) S.pbar_phase = ph0 + (unsigned)(n - 1);
   }
-  // balls that end at the window's last plane: every layer's open partial (a
-  // layer with no ball there writes a zero no reduction reads); then every
+  // balls that end at the window's last plane: the open partials; then every
   // ball's columns are summed
-  if (tv) {
 #pragma unroll
-    for (int j = 0; j < RY; j++) {
-      if (!ok[j]) continue;
+  for (int j = 0; j < RY; j++) {
+    if (!ok[j]) continue;
 #pragma unroll
-      for (int k = 0; k < KL; k++) {
+    for (int k = 0; k < KL; k++) {
 #pragma unroll
-        for (int q = 0; q < PM; q++) fb[((k * PM + q) * n + n - 1) * n2 + col[j]] = acd[j][k][q];
-        if constexpr (IND) fbw[(k * n + n - 1) * n2 + col[j]] = accw[(k * RY + j) * NS + tid];
+      for (int i = 0; i < 2; i++) {
+        if (lay_of(idc[j][i], k) == dummy) continue;
+        const int f = (k * PM * n + n - 1) * VP + g0 + j * NP + i;
+#pragma unroll
+        for (int q = 0; q < PM; q++) fb[f + q * NW] = i ? acd[j][k][q].y : acd[j][k][q].x;
+        if constexpr (IND) fb[f + fset] = i ? acw[j][k].y : acw[j][k].x;
       }
     }
   }
   bar_sweep(NS);
-  for (int p = warp; p < S.n_pi; p += nwarp) reduce_instance<PM, IND>(a, S, fb, p, lane);
+  reduce_instances<PM, IND>(a, S, fb, warp, nwarp, lane);
   bar_sweep(NS);
 }
 
@@ -635,25 +747,29 @@ static __device__ void sweep_sum2(Shared &S, double v0, double v1, int NS) {
 // which leaves every sign and rounding unchanged.  An exact zero counts as
 // positive (a test point on an eigenvalue of a leading submatrix; the
 // multisection's brackets tolerate the one-off count there).
-static __device__ int sturm_count(const double *d, const double *e, int m, double x) {
+static __device__ int sturm_count(const double *d, const double *e2, int m, double x) {
   double p0 = 1.0, p1 = d[0] - x;
   int cnt = p1 < 0.0;
-  for (int i = 1; i < m; i++) {
-    const double p2 = (d[i] - x) * p1 - (e[i - 1] * e[i - 1]) * p0;
+  int i = 1;
+  auto row = [&](int r) {
+    const double p2 = (d[r] - x) * p1 - e2[r - 1] * p0;
     cnt += (p2 < 0.0) != (p1 < 0.0);
     p0 = p1;
     p1 = p2;
-    if ((i & 7) == 0) {
-      const double mx = fmax(fabs(p0), fabs(p1));
-      if (mx > 0x1p+600) {
-        p0 *= 0x1p-600;
-        p1 *= 0x1p-600;
-      } else if (mx < 0x1p-600 && mx > 0.0) {
-        p0 *= 0x1p+600;
-        p1 *= 0x1p+600;
-      }
+  };
+  for (; i + 8 <= m; i += 8) {
+#pragma unroll
+    for (int r = 0; r < 8; r++) row(i + r);
+    const double mx = fmax(fabs(p0), fabs(p1));
+    if (mx > 0x1p+600) {
+      p0 *= 0x1p-600;
+      p1 *= 0x1p-600;
+    } else if (mx < 0x1p-600 && mx > 0.0) {
+      p0 *= 0x1p+600;
+      p1 *= 0x1p+600;
     }
   }
+  for (; i < m; i++) row(i);
   return cnt;
 }
 
@@ -668,31 +784,28 @@ static __device__ void tridiag_extremes(Shared &S, int m) {
   const int G = nw / 2, N = 32 * G;
   const int g = warp < G ? 0 : (warp < 2 * G ? 1 : 2);
   const int gi = warp - g * G;
+  // Gershgorin interval: the complete rows' part is kept by lanczos, the last
+  // row has one neighbour.  Warm start from the previous (one row smaller)
+  // tridiagonal's extremes: by interlacing the new smallest lies at or below
+  // the old one and the new largest at or above it; the other end of each
+  // bracket is the old extreme moved by four times its last change, which the
+  // first round tests beside its inner points.
+  const double rl = m > 1 ? fabs(S.bb[m - 2]) : 0.0;
+  double glo = fmin(S.ger[0], S.aa[m - 1] - rl), ghi = fmax(S.ger[1], S.aa[m - 1] + rl);
+  const double span = fmax(fabs(glo), fabs(ghi));
+  glo -= 1e-14 * span + 1e-300;
+  ghi += 1e-14 * span + 1e-300;
+  bool first = S.warm != 0;
   if (tid == 0) {
-    const double *d = S.aa, *e = S.bb;
-    double lo = 1e300, hi = -1e300;
-    for (int i = 0; i < m; i++) {
-      const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < m - 1 ? fabs(e[i]) : 0.0);
-      lo = fmin(lo, d[i] - r);
-      hi = fmax(hi, d[i] + r);
-    }
-    const double span = fmax(fabs(lo), fabs(hi));
-    lo -= 1e-14 * span + 1e-300;
-    hi += 1e-14 * span + 1e-300;
-    S.br[0][0] = S.br[1][0] = lo;
-    S.br[0][1] = S.br[1][1] = hi;
-    if (S.warm) {
-      // Warm start from the previous (one row smaller) tridiagonal's extremes:
-      // by interlacing the new smallest lies at or below the old one and the
-      // new largest at or above it; the other end of each bracket is the old
-      // extreme moved by four times its last change, kept when a Sturm count
-      // confirms that no eigenvalue lies beyond it.
+    S.br[0][0] = S.br[1][0] = glo;
+    S.br[0][1] = S.br[1][1] = ghi;
+    if (first) {
       const double pad = 16.0 * 2.220446049250313e-16 * span;
       const double x0 = S.eig[0] - fmax(4.0 * S.wdel[0], 1e-9 * span), x1 = S.eig[1] + fmax(4.0 * S.wdel[1], 1e-9 * span);
-      if (S.eig[0] + pad < hi) S.br[0][1] = S.eig[0] + pad;
-      if (x0 > lo && sturm_count(d, e, m, x0) == 0) S.br[0][0] = x0;
-      if (S.eig[1] - pad > lo) S.br[1][0] = S.eig[1] - pad;
-      if (x1 < hi && sturm_count(d, e, m, x1) == m) S.br[1][1] = x1;
+      if (S.eig[0] + pad < ghi) S.br[0][1] = S.eig[0] + pad;
+      if (S.eig[1] - pad > glo) S.br[1][0] = S.eig[1] - pad;
+      S.br[0][0] = fmax(x0, glo);
+      S.br[1][1] = fmin(x1, ghi);
     }
   }
   __syncthreads();
@@ -701,12 +814,17 @@ static __device__ void tridiag_extremes(Shared &S, int m) {
     return hi - lo > 4.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + 1e-300;
   };
   for (int it = 0; it < 80; it++) {
-    const bool a0 = active(0), a1 = active(1);
+    const bool a0 = first || active(0), a1 = first || active(1);
     if (!a0 && !a1) break;
+    // points of a round: lo + w i / (N + 1), i = 1 .. N; in a warm first round
+    // the guessed end is a point too: i = 0 .. N - 1 for the smallest (lo
+    // guessed), i = 2 .. N + 1 for the largest (hi guessed)
+    const int sh = first ? (g == 0 ? -1 : 1) : 0;
+    const double inv = 1.0 / (double)(N + 1);
     if (g < 2 && (g == 0 ? a0 : a1)) {
       const double lo = S.br[g][0], w = S.br[g][1] - lo;
-      const int i = gi * 32 + lane;
-      const int c = sturm_count(S.aa, S.bb, m, lo + w * (double)(i + 1) / (double)(N + 1));
+      const int i = gi * 32 + lane, j = i + 1 + sh;
+      const int c = sturm_count(S.aa, S.b2, m, j == N + 1 ? S.br[g][1] : lo + w * ((double)j * inv));
       if (g == 0) {
         const unsigned below = __ballot_sync(0xffffffffu, c >= 1);
         if (lane == 0) S.wres[warp] = below ? gi * 32 + __ffs(below) - 1 : N;
@@ -716,31 +834,25 @@ static __device__ void tridiag_extremes(Shared &S, int m) {
       }
     }
     __syncthreads();
-    if (tid == 0) {
-      const double inv = 1.0 / (double)(N + 1);
-      if (a0) {  // smallest: the first point with an eigenvalue below it
+    if (tid < 2 && (tid == 0 ? a0 : a1)) {
+      const double lo = S.br[tid][0], hi = S.br[tid][1], w = hi - lo;
+      if (tid == 0) {  // smallest: the first point with an eigenvalue below it
+        const int s0 = first ? -1 : 0;
         int f = N;
-        for (int w = 0; w < G; w++) f = min(f, S.wres[w]);
-        const double lo = S.br[0][0], w = S.br[0][1] - lo;
-        if (f == N) {
-          S.br[0][0] = lo + w * (double)N * inv;
-        } else {
-          S.br[0][1] = lo + w * (double)(f + 1) * inv;
-          if (f > 0) S.br[0][0] = lo + w * (double)f * inv;
-        }
-      }
-      if (a1) {  // largest: the last point with an eigenvalue above it
+        for (int v = 0; v < G; v++) f = min(f, S.wres[v]);
+        if (f < N) S.br[0][1] = f + 1 + s0 == 0 ? lo : lo + w * ((double)(f + 1 + s0) * inv);
+        if (f > 0) S.br[0][0] = f + s0 == 0 ? lo : lo + w * ((double)(f + s0) * inv);
+        else if (first) S.br[0][0] = glo;  // an eigenvalue lies below the guess
+      } else {  // largest: the last point with an eigenvalue above it
+        const int s1 = first ? 1 : 0;
         int l = -1;
-        for (int w = 0; w < G; w++) l = max(l, S.wres[G + w]);
-        const double lo = S.br[1][0], w = S.br[1][1] - lo;
-        if (l < 0) {
-          S.br[1][1] = lo + w * inv;
-        } else {
-          if (l < N - 1) S.br[1][1] = lo + w * (double)(l + 2) * inv;
-          S.br[1][0] = lo + w * (double)(l + 1) * inv;
-        }
+        for (int v = 0; v < G; v++) l = max(l, S.wres[G + v]);
+        if (l >= 0) S.br[1][0] = l + 1 + s1 == N + 1 ? hi : lo + w * ((double)(l + 1 + s1) * inv);
+        if (l < N - 1) S.br[1][1] = l + 2 + s1 == N + 1 ? hi : lo + w * ((double)(l + 2 + s1) * inv);
+        else if (first) S.br[1][1] = ghi;  // an eigenvalue lies above the guess
       }
     }
+    first = false;
     __syncthreads();
   }
   if (tid == 0) {
@@ -872,6 +984,27 @@ static __device__ void count_proj_points(const SweepArgs &a, Shared &S, long lon
   atomicAdd(a.proj_points + 2, win * (unsigned long long)steps);
 }
 
+// The node's unit vector e_c, and the scaled Lanczos start vector, into a
+// window vector (pad columns zero).
+template <typename T>
+static __device__ void unit_vector(const SweepArgs &a, Shared &S, T *v) {
+  const int NP = pair_cols(a.n), nw = (int)vec_points(a.n), nl = a.nloc;
+  const int c = (nl * a.n + nl) * NP + nl + (S.gi & 1);
+  __syncthreads();
+  for (int i = threadIdx.x; i < nw; i += blockDim.x) v[i] = (T)(i == c ? 1.0 : 0.0);
+  __syncthreads();
+}
+template <typename T>
+static __device__ void start_vector(const SweepArgs &a, Shared &S, T *v, double scale) {
+  const int n = a.n, NP = pair_cols(n), nw = (int)vec_points(n), sh = S.gi & 1;
+  __syncthreads();
+  for (int i = threadIdx.x; i < nw; i += blockDim.x) {
+    const int row = i / NP, x = i - row * NP - sh;  // row = z n + y, of the parity of z + y
+    v[i] = (T)(x >= 0 && x < n ? scale * start_val(a.lz_chk, row + x) : 0.0);
+  }
+  __syncthreads();
+}
+
 // Lanczos bounds (sq.cpp:965-1092) in storage precision T, or (LQ) bounds and
 // moments from one FP64 Lanczos run started at e_c.  Sweep m applies H to the
 // unnormalised W_m = w_m-1 (v_m = s_m W_m), formed while it is loaded from the
@@ -881,7 +1014,7 @@ static __device__ void count_proj_points(const SweepArgs &a, Shared &S, long lon
 // extremes moved by no more than the tolerance, at most 500 steps) applies.
 // The projections chi^T W_m+1 the next gather needs follow from the recurrence
 // on the dot products of the sweep's output.
-template <typename T, int PM, bool LQ, int RY>
+template <typename T, int PM, bool LQ, int RY, int NT>
 __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, double *pcur, double &lmin_out,
                         double &lmax_out, int &rows_out) {
   const int tid = threadIdx.x;
@@ -893,13 +1026,15 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
   const int kmin = a.npl / 2 + 1;
   double d0 = 0.0, d1 = 0.0;
   if constexpr (LQ) {
+    unit_vector(a, S, Y);
     centre_projections(a, S, pcur);  // W_0 = e_c
   } else {
+    start_vector(a, S, Y, s0);
     // chi^T W_0 for W_0 = (1 + chk (-1)^(x+y+z)) / norm (sq.cpp:538-546, 993-1004
     // with chk = 0)
     IO<T> io;
     io.chk = chk;
-    sweep<T, PM, SK_ONES, RY>(a, S, dyn, io, d0, d1);
+    sweep<T, PM, SK_ONES, RY, NT>(a, S, dyn, io, d0, d1);
     __syncthreads();
     for (int p = tid; p < S.n_pi; p += blockDim.x) {
       S.pw_cur[p] = s0 * S.p_nxt[p];
@@ -912,6 +1047,8 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
     S.count = 0;
     S.eprev[0] = S.eprev[1] = 0.0;
     S.warm = 0;
+    S.ger[0] = 1e300;
+    S.ger[1] = -1e300;
   }
   __syncthreads();
   double a_prev = 0.0, s_prev = 1.0, bs_prev = 0.0;
@@ -919,10 +1056,8 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
     IO<T> io;
     io.out = Y;
     io.wout = Wv[m & 1];
-    if (m == 0) {
-      io.konst = LQ ? 2 : 1;
-      io.chk = chk;
-      io.sin = s0;
+    if (m == 0) {  // W_0 = 1 (Y - 0 W1) - 0 W2 from the start vector in Y
+      io.vin = io.p1 = io.p2 = Y;
     } else {
       io.vin = Y;
       io.p1 = Wv[(m - 1) & 1];
@@ -933,7 +1068,7 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
     }
     d0 = 0.0;
     d1 = 0.0;
-    sweep<T, PM, SK_LZF, RY>(a, S, dyn, io, d0, d1);
+    sweep<T, PM, SK_LZF, RY, NT>(a, S, dyn, io, d0, d1);
     sweep_sum2(S, d0, d1, a.nsweep);
     // b_m-1 = |W_m| and a_m = <W_m, H W_m> / b_m-1^2 (W_0 is normalised)
     const double bm = m == 0 ? 1.0 : sqrt(S.scal[0]);
@@ -941,7 +1076,13 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
     const double sm = 1.0 / bm;
     if (tid == 0) {
       S.aa[m] = am;
-      if (m > 0) S.bb[m - 1] = bm;
+      if (m > 0) {
+        S.bb[m - 1] = bm;
+        S.b2[m - 1] = bm * bm;
+        const double r = bm + (m > 1 ? S.bb[m - 2] : 0.0);  // row m - 1 is complete
+        S.ger[0] = fmin(S.ger[0], S.aa[m - 1] - r);
+        S.ger[1] = fmax(S.ger[1], S.aa[m - 1] + r);
+      }
     }
     __syncthreads();
     // after sweep m the tridiagonal has m + 1 rows (complete from m = 1; the
@@ -997,20 +1138,21 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
 }
 
 // Chebyshev moments mu_j = e_c^T T_j((H - chi)/zee) e_c / h^3 (sq.cpp:564-655).
-template <int PM, int RY>
+template <int PM, int RY, int NT>
 __device__ void moments(const SweepArgs &a, Shared &S, unsigned char *dyn, double *pcur, double chi, double zee,
                         double *mu) {
   double *B0 = slot<double>(a, 0), *B1 = slot<double>(a, 1);
   double d0 = 0.0, d1 = 0.0;
   centre_projections(a, S, pcur);
+  unit_vector(a, S, B0);
   {  // t_1 = (H e_c - chi e_c) / zee
     IO<double> io;
-    io.konst = 2;
+    io.vin = B0;
     io.first = 1;
     io.out = B1;
     io.ca = chi;
     io.cb = zee;
-    sweep<double, PM, SK_CH, RY>(a, S, dyn, io, d0, d1);
+    sweep<double, PM, SK_CH, RY, NT>(a, S, dyn, io, d0, d1);
   }
   __syncthreads();
   rotate(S, pcur);
@@ -1026,14 +1168,13 @@ __device__ void moments(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
       IO<double> io;
       io.vin = t1;
       io.p1 = t0;
-      io.p1_delta = nq == 2;  // t_0 = e_c
       io.out = t0;
       io.ca = chi;
       io.cb = zee;
       io.dbl = nq > q1;
       d0 = 0.0;
       d1 = 0.0;
-      sweep<double, PM, SK_CH, RY>(a, S, dyn, io, d0, d1);
+      sweep<double, PM, SK_CH, RY, NT>(a, S, dyn, io, d0, d1);
       if (nq > q1) sweep_sum2(S, d0, d1, a.nsweep);
     }
     __syncthreads();
@@ -1086,16 +1227,17 @@ static __device__ void sweep_sum3(Shared &S, double v0, double v1, double v2) {
 // of D (zero outside the window) contracted with the replica's projectors:
 // f = -4 h^3 sum_q (chi_q . grad D) chi_q(centre) / Denom_q, into the node's
 // force slots (atom, fx, fy, fz).
-template <typename T, int PM, int RY>
+template <typename T, int PM, int RY, int NT>
 __device__ void node_forces(const SweepArgs &a, Shared &S, unsigned char *dyn, double *pcur, double chi,
                             double zee, const double *ci, double *fslot) {
   T *B0 = slot<T>(a, 0), *B1 = slot<T>(a, 1);
   double *D = slot<double>(a, 2);
   double d0 = 0.0, d1 = 0.0;
+  unit_vector(a, S, B0);
   centre_projections(a, S, pcur);
   {  // t_1 = (H e_c - chi e_c) / zee; D = e_c Ci_0 / h^3 + t_1 Ci_1 / h^3
     IO<T> io;
-    io.konst = 2;
+    io.vin = B0;
     io.first = 1;
     io.out = B1;
     io.ca = chi;
@@ -1103,7 +1245,7 @@ __device__ void node_forces(const SweepArgs &a, Shared &S, unsigned char *dyn, d
     io.dacc = D;
     io.ce = ci[0];
     io.cd = ci[1];
-    sweep<T, PM, SK_FD, RY>(a, S, dyn, io, d0, d1);
+    sweep<T, PM, SK_FD, RY, NT>(a, S, dyn, io, d0, d1);
   }
   __syncthreads();
   rotate(S, pcur);
@@ -1112,13 +1254,12 @@ __device__ void node_forces(const SweepArgs &a, Shared &S, unsigned char *dyn, d
     IO<T> io;
     io.vin = t1;
     io.p1 = t0;
-    io.p1_delta = nq == 2;  // t_0 = e_c
     io.out = t0;
     io.ca = chi;
     io.cb = zee;
     io.dacc = D;
     io.cd = ci[nq];
-    sweep<T, PM, SK_FD, RY>(a, S, dyn, io, d0, d1);
+    sweep<T, PM, SK_FD, RY, NT>(a, S, dyn, io, d0, d1);
     __syncthreads();
     rotate(S, pcur);
     T *tt = t0;
@@ -1127,7 +1268,7 @@ __device__ void node_forces(const SweepArgs &a, Shared &S, unsigned char *dyn, d
   }
   __threadfence_block();
   __syncthreads();
-  const int n = a.n, nl = a.nloc, n2 = n * n, EV = (int)a.evol;
+  const int n = a.n, nl = a.nloc, NP = pair_cols(n), VP = n * NP, sh = S.gi & 1, EV = (int)a.evol;
   int slotc = 0;
   for (int e = 0; e < S.n_ent; e++) {
     if (nl < S.e_x0[e] || nl > S.e_x1[e] || nl < S.e_y0[e] || nl > S.e_y1[e] || nl < S.e_z0[e] || nl > S.e_z1[e])
@@ -1141,12 +1282,12 @@ __device__ void node_forces(const SweepArgs &a, Shared &S, unsigned char *dyn, d
       double ax = 0.0, ay = 0.0, az = 0.0;
       for (int i = threadIdx.x; i < vol; i += blockDim.x) {
         const int x = x0 + i % bx, y = y0 + (i / bx) % by, z = z0 + i / (bx * by);
-        const int w = SQB_IDX(z * n2 + y * n + x, n * n2, a.status);
+        const int w = SQB_IDX(z * VP + y * NP + x + sh, n * VP, a.status);
         double gx = 0.0, gy = 0.0, gz = 0.0;
         for (int kk = 1; kk <= FDN; kk++) {
           const double xm = x - kk >= 0 ? D[w - kk] : 0.0, xp = x + kk < n ? D[w + kk] : 0.0;
-          const double ym = y - kk >= 0 ? D[w - kk * n] : 0.0, yp = y + kk < n ? D[w + kk * n] : 0.0;
-          const double zm = z - kk >= 0 ? D[w - kk * n2] : 0.0, zp = z + kk < n ? D[w + kk * n2] : 0.0;
+          const double ym = y - kk >= 0 ? D[w - kk * NP] : 0.0, yp = y + kk < n ? D[w + kk * NP] : 0.0;
+          const double zm = z - kk >= 0 ? D[w - kk * VP] : 0.0, zp = z + kk < n ? D[w + kk * VP] : 0.0;
           gx += (-xm + xp) * a.coeff_grad[kk];
           gy += (-ym + yp) * a.coeff_grad[kk];
           gz += (-zm + zp) * a.coeff_grad[kk];
@@ -1181,15 +1322,15 @@ __device__ void node_forces(const SweepArgs &a, Shared &S, unsigned char *dyn, d
 }
 
 // The force pass over the listed nodes (bounds from chi, zee; Ci from ci).
-template <int PM, typename T, int MAXT, int RY>
-__global__ void __launch_bounds__(MAXT, 1) sweep_force_kernel(SweepArgs a) {
+template <int PM, typename T, int MAXT, int RY, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) sweep_force_kernel(SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   Shared &S = *reinterpret_cast<Shared *>(smem);
   unsigned char *dyn = smem + shared_fixed();
-  double *pcur =
-      reinterpret_cast<double *>(dyn + planes_bytes(a.n, RY) + ring_bytes(a.nsweep, PM, RY) + accw_bytes(a.nsweep, PM, RY));
+  double *pcur = reinterpret_cast<double *>(dyn + planes_bytes(a.n, RY) + ring_bytes(MAXT, RY));
   for (int i = threadIdx.x; i < a.n_gproj + PM; i += blockDim.x) pcur[i] = 0.0;  // [n_gproj..]: the empty id
   pbar_setup(S);
+  zero_planes(a, dyn, RY);
   for (;;) {
     if (threadIdx.x == 0) {
       const int q = atomicAdd(a.counter, 1);
@@ -1207,7 +1348,7 @@ __global__ void __launch_bounds__(MAXT, 1) sweep_force_kernel(SweepArgs a) {
     double *fs = a.fslots + (size_t)S.qidx * FSLOTS * 4;
     for (int i = threadIdx.x; i < FSLOTS * 4; i += blockDim.x) fs[i] = (i % 4 == 0) ? -1.0 : 0.0;
     setup_node(a, S);
-    node_forces<T, PM, RY>(a, S, dyn, pcur, a.chi[node], a.zee[node], a.ci + (size_t)node * (a.npl + 1), fs);
+    node_forces<T, PM, RY, MAXT>(a, S, dyn, pcur, a.chi[node], a.zee[node], a.ci + (size_t)node * (a.npl + 1), fs);
     __syncthreads();
   }
 }
@@ -1246,15 +1387,15 @@ static __device__ void quadrature_moments(const SweepArgs &a, Shared &S, int k, 
 
 // FORM: 0 FP64, 1 FP32-mixed, 2 Lanczos quadrature.  MAXT bounds the block,
 // which sets the register budget per thread.
-template <int PM, int FORM, int MAXT, int RY>
-__global__ void __launch_bounds__(MAXT, 1) sweep_kernel(SweepArgs a) {
+template <int PM, int FORM, int MAXT, int RY, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) sweep_kernel(SweepArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   Shared &S = *reinterpret_cast<Shared *>(smem);
   unsigned char *dyn = smem + shared_fixed();
-  double *pcur =
-      reinterpret_cast<double *>(dyn + planes_bytes(a.n, RY) + ring_bytes(a.nsweep, PM, RY) + accw_bytes(a.nsweep, PM, RY));
+  double *pcur = reinterpret_cast<double *>(dyn + planes_bytes(a.n, RY) + ring_bytes(MAXT, RY));
   for (int i = threadIdx.x; i < a.n_gproj + PM; i += blockDim.x) pcur[i] = 0.0;  // [n_gproj..]: the empty id
   pbar_setup(S);
+  zero_planes(a, dyn, RY);
   for (;;) {
     if (threadIdx.x == 0) {
       const int q = atomicAdd(a.counter, 1);
@@ -1274,7 +1415,7 @@ __global__ void __launch_bounds__(MAXT, 1) sweep_kernel(SweepArgs a) {
     int rows = 0;
     double *mu = a.rho_pj + (size_t)node * (a.npl + 1);
     if constexpr (FORM == 2) {
-      lanczos<double, PM, true, RY>(a, S, dyn, pcur, lmin, lmax, rows);
+      lanczos<double, PM, true, RY, MAXT>(a, S, dyn, pcur, lmin, lmax, rows);
       const double chi = 0.5 * (lmax + lmin), zee = 0.5 * (lmax - lmin);
       if ((long long)rows <= (long long)a.n * a.n * a.n) quadrature_moments(a, S, rows, chi, zee, mu);
       else if (threadIdx.x == 0) atomicOr(a.status, ST_CAPACITY);
@@ -1282,12 +1423,14 @@ __global__ void __launch_bounds__(MAXT, 1) sweep_kernel(SweepArgs a) {
       rows -= 1;  // reported as Lanczos iterations: matvecs = iterations + 1
     } else {
       using TL = typename std::conditional<FORM == 1, float, double>::type;
-      lanczos<TL, PM, false, RY>(a, S, dyn, pcur, lmin, lmax, rows);
+      if (FORM == 1) zero_planes(a, dyn, RY);  // FP32 values next
+      lanczos<TL, PM, false, RY, MAXT>(a, S, dyn, pcur, lmin, lmax, rows);
       const double chi = (lmax + lmin) / 2, zee = (lmax - lmin) / 2;  // sq.cpp:564-565
       count_proj_points(a, S, rows + 1, 0);
       // moments stay FP64 in both forms: FP32 storage of the Chebyshev vectors
       // grows a rounding error injected at step i like (k - i) by step k
-      moments<PM, RY>(a, S, dyn, pcur, chi, zee, mu);
+      if (FORM == 1) zero_planes(a, dyn, RY);  // FP64 values next
+      moments<PM, RY, MAXT>(a, S, dyn, pcur, chi, zee, mu);
       count_proj_points(a, S, a.npl / 2, 1);
     }
     if (threadIdx.x == 0) {
@@ -1300,6 +1443,34 @@ __global__ void __launch_bounds__(MAXT, 1) sweep_kernel(SweepArgs a) {
     __syncthreads();
   }
 }
+
+// Tiles: rows per thread and the launch bound, which sets the registers per
+// thread.  One row per thread by default: two rows share their y-arm loads and
+// issue 20% fewer instructions per point, but their 8 warps of 255 registers
+// hide less latency than 16 warps of 128 (B200, 288 nodes of 31^3 windows,
+// FP64: 25.4 against 20.8 ms; 27^3: 23.4 against 16.6 ms; 39^3, 13 against 25
+// warps: the same).  Windows up to 19 wide keep two CTAs on an SM at least.
+constexpr int TILE_N_MAX = 43;    // widest window of the default tiles
+constexpr int TILE_N_ROWS3 = 33;  // and of three rows per thread
+// Launch bound of the tile (and the ring's stride).
+inline int tile_bound(int n, int ry) {
+  const int t = sweep_threads_of(n, ry);
+  return ry == 3 ? 192 : t <= 192 ? 192 : t <= 384 ? 384 : t <= 512 ? 512 : t <= 640 ? 640 : 1024;
+}
+template <class K>
+const void *pick_tile(int n, int ry) {
+  if (ry == 3) return n <= TILE_N_ROWS3 ? K::template get<192, 3, 1>() : nullptr;
+  if (ry != 1 || n > TILE_N_MAX) return nullptr;
+  const int m = tile_bound(n, ry);
+  return m == 192   ? K::template get<192, 1, 2>()
+         : m == 384 ? K::template get<384, 1, 1>()
+         : m == 512 ? K::template get<512, 1, 1>()
+         : m == 640 ? K::template get<640, 1, 1>()
+                    : K::template get<1024, 1, 1>();
+}
+// Shared-memory limit of a kernel for this launch and, on request, its
+// resident CTAs per SM.
+cudaError_t tile_setup(const void *kernel, const SweepArgs &a, int *per_sm);
 
 }  // namespace sweep
 }  // namespace sqb

@@ -1,0 +1,75 @@
+"""The sweep kernel's tiles and layers against the plane-streaming kernel, at the sizes
+where they can go wrong.
+
+The window edges are the smallest and largest of every tile (pairs of columns: windows
+that start at odd and even columns of the halo'd block, the last pair half outside), for
+fields with one and with three projectors per slot.  Both kernels sum in FP64 in another
+order: a moment of order k carries about k^2 roundings of size 1e-16 (npl 16: 1e-13 with
+room), the bounds 1e-12 of the spectral range.  With three projectors per slot both
+kernels carry the projections of a Lanczos step by recurrence, whose rounding grows with
+the step count, so their bounds agree only within the stop: 1e-6 Ha of about 35 Ha, 3e-8,
+and the moments ten times that.  FP32 Lanczos vectors round at 6e-8, and
+the stop at 1e-3 Ha is met within that of each other.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return float(np.abs(a - b).max() / max(np.abs(b).max(), 1e-300))
+
+
+def _params(kind, system, nloc, form=0, npl=16, **kw):
+    d = dict(kind=kind, system=system, form=form, cells=2, per_cell=12 if nloc < 14 else 20, block="3x2x2",
+             nloc=nloc, npl=npl, kt=5.0)
+    d.update(kw)
+    return d
+
+
+def _both(p, seed=3):
+    """Outputs of the sweep kernel and of the plane-streaming kernel on the same inputs."""
+    from perf import cases
+    from sqdft_b200 import sq
+
+    s = cases.prepare(p, seed)
+    with s["ctx"] as ctx:
+        ctx.set_node_kernel(sq.SQB_KERNEL_SWEEP)
+        a = cases.run(s)
+        ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
+        return a, cases.run(s)
+
+
+@pytest.mark.parametrize("system", ["al", "lih"])
+@pytest.mark.parametrize("nloc", [4, 9, 10, 13, 15, 16, 17, 19, 21])
+def test_tiles_match_plane_kernel(system, nloc):
+    if system == "lih" and nloc == 9:
+        pytest.skip("two species at this spacing need more than four layers")
+    for form in (0, 1, 2):
+        a, b = _both(_params("sq", system, nloc, form, per_cell=20 if system == "lih" or nloc > 13 else 12))
+        tol = 1e-6 if form == 1 else 3e-8 if system == "lih" else 1e-12
+        for k in ("chi", "zee"):
+            assert _rel(a[k], b[k]) <= tol, (form, k)
+        assert _rel(a["rho_pj"], b["rho_pj"]) <= 10 * tol, form
+    for form in (0, 1):
+        a, b = _both(_params("forces", system, nloc, form, per_cell=20 if system == "lih" or nloc > 13 else 12))
+        assert _rel(a, b) <= (1e-5 if form else 1e-11), form
+
+
+def test_layers_of_displaced_lih_fit():
+    """Displaced 64-atom LiH, where first fit in replica order needs five or six layers."""
+    from perf import cases
+    from sqdft_b200 import sq
+
+    p = _params("sq", "lih", 16, per_cell=20, npl=16, block="6x5x4")
+    for seed in (0, 1, 2):
+        s = cases.prepare(p, seed)
+        with s["ctx"] as ctx:
+            a = cases.run(s)
+            assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_SWEEP
+            ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
+            b = cases.run(s)
+        assert _rel(a["rho_pj"], b["rho_pj"]) <= 3e-7
