@@ -402,14 +402,12 @@ int ensure_layers(sqb_ctx *c) {
   CK(cudaMemcpy(off_all.data(), c->d_rep_off, off_all.size() * sizeof(long long), cudaMemcpyDeviceToHost));
   std::vector<long long> off(std::max<size_t>(boxes.size(), 1));
   for (size_t i = 0; i < boxes.size(); i++) off[i] = off_all[boxes[i].r];
-  long long *d_off = nullptr;
-  CK(cudaMalloc((void **)&d_off, off.size() * sizeof(long long)));
-  CK(cudaMemcpy(d_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice));
-  const cudaError_t e = launch_fill_layers((int)boxes.size(), c->d_rep_box, c->d_rep_gpb, c->d_typ_nlocc, d_off,
+  CK(dalloc(&c->d_rep_off_l, off.size()));
+  CK(cudaMemcpy(c->d_rep_off_l, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice));
+  const cudaError_t e = launch_fill_layers((int)boxes.size(), c->d_rep_box, c->d_rep_gpb, c->d_typ_nlocc, c->d_rep_off_l,
                                            c->d_tab64, c->ex, c->ey, c->ez, c->exp, pm, ngp, c->d_lay_id, c->d_lay_chi,
                                            c->stream);
   const cudaError_t e2 = cudaStreamSynchronize(c->stream);
-  cudaFree(d_off);
   CK(e);
   CK(e2);
   c->lay_state = 1;
@@ -1835,17 +1833,46 @@ static int moments_vjp(sqb_ctx *c, Fill fill, double *g_veff, double *g_atoms) {
   const size_t nw = (size_t)c->n * c->n * c->n;
   const size_t ext = (size_t)c->ex * c->ey * c->ez;
   const int nseg = (c->g.npl + VJP_K - 1) / VJP_K;
-  const size_t per = ((size_t)(2 * nseg + VJP_K + 4) * nw + (size_t)nseg * MAXP + 31) & ~size_t(31);  // doubles
+  size_t per = ((size_t)(2 * nseg + VJP_K + 4) * nw + (size_t)nseg * MAXP + 31) & ~size_t(31);  // doubles
   int grid = c->sms * (c->ctas_per_sm > 0 ? c->ctas_per_sm : 1);
   if ((size_t)grid > N) grid = (int)N;
-  const size_t need = (per * grid + N * K + ext) * sizeof(double);
-  if (c->vjp_bytes < need) {
+  auto reserve = [&](size_t need) {
+    if (c->vjp_bytes >= need) return true;
     if (c->d_vjp) cudaFree(c->d_vjp);
     c->d_vjp = nullptr;
     c->vjp_bytes = 0;
-    CK(cudaMalloc((void **)&c->d_vjp, need));
+    if (cudaMalloc((void **)&c->d_vjp, need) != cudaSuccess) {
+      cudaGetLastError();
+      c->d_vjp = nullptr;
+      return false;
+    }
     c->vjp_bytes = need;
+    return true;
+  };
+  // The sweep kernel where it covers the system and its npl window vectors per
+  // CTA can be had (27^3 windows, npl 64: 1.5 GB in all; the plane-streaming
+  // kernel's checkpoints take 0.6 GB and its reverse recursion three times the
+  // matvecs), else the plane-streaming kernel.
+  int rc = c->node_kernel == SQB_KERNEL_PLANE ? SQB_OK : ensure_layers(c);
+  if (rc) return rc;
+  bool sw = c->node_kernel != SQB_KERNEL_PLANE && c->lay_state == 1;
+  SweepArgs sa;
+  if (sw) {
+    fill_sweep_args(c, c->d_nodes, c->nnode, sa);
+    int per_sm = 0;
+    CK(sweep_vjp_per_sm(sa, &per_sm));
+    const int g = std::max(1, std::min(c->sms * per_sm, c->nnode));
+    const size_t p = sweep_vjp_doubles(c->n, c->g.npl);
+    sw = reserve((p * g + N * K + ext) * sizeof(double));
+    if (sw) {
+      grid = g;
+      per = p;
+      rc = ensure_sweep_scratch(c, grid, &sa.scratch_stride);
+      if (rc) return rc;
+      sa.scratch = c->d_scratch;
+    }
   }
+  if (!sw && !reserve((per * grid + N * K + ext) * sizeof(double))) return SQB_ERR_CUDA;
   double *d_scr = c->d_vjp, *d_g = d_scr + per * grid, *d_out = d_g + N * K;
   const size_t per_at = (size_t)(4 * VJP_K + 12) * MAXP;  // doubles per CTA
   double *d_gat = nullptr;
@@ -1863,7 +1890,7 @@ static int moments_vjp(sqb_ctx *c, Fill fill, double *g_veff, double *g_atoms) {
     d_gat = c->d_vjp_at + per_at * grid;
     CK(cudaMemsetAsync(d_gat, 0, (size_t)3 * std::max(c->n_atm, 1) * sizeof(double), c->stream));
   }
-  int rc = fill(d_g);
+  rc = fill(d_g);
   if (rc) return rc;
   CK(cudaMemsetAsync(d_out, 0, ext * sizeof(double), c->stream));
   NodeArgs a;
@@ -1883,8 +1910,26 @@ static int moments_vjp(sqb_ctx *c, Fill fill, double *g_veff, double *g_atoms) {
     a.vjp_at_stride = per_at;
   }
   CK(cudaEventRecord(c->ev0, c->stream));
-  rc = run_nodes(c, a, c->d_nodes, c->nnode);
-  if (rc) return rc;
+  if (sw) {
+    sa.chi = c->d_chi;
+    sa.zee = c->d_zee;
+    sa.gmu = d_g;
+    sa.vjp = d_scr;
+    sa.vjp_stride = per;
+    sa.g_veff = d_out;
+    sa.gex = c->ex;
+    sa.dtab = a.dtab;
+    sa.dtab_stride = a.dtab_stride;
+    sa.rep_off = c->d_rep_off_l;
+    sa.g_atoms = a.g_atoms;
+    CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->d_proj_points, 0, 3 * sizeof(unsigned long long), c->stream));
+    CK(launch_sweep_vjp(sa, grid, c->stream));
+  } else {
+    rc = run_nodes(c, a, c->d_nodes, c->nnode);
+    if (rc) return rc;
+  }
   CK(cudaEventRecord(c->ev1, c->stream));
   rc = read_status(c);
   c->stats.ms_vjp = elapsed(c);

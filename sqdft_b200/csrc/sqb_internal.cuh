@@ -171,6 +171,20 @@ struct SweepArgs {
   double coeff_grad[FDN + 1];
   const int *rep_atom;
   double *fslots;
+  // adjoint (sweep_vjp_kernel): bounds in chi, zee (inputs), the weights dL/dmu
+  // [node][npl+1], per-CTA scratch, dL/dVeff on the halo'd block (rows of gex
+  // values, accumulated with atomics); with g_atoms the derivative tables
+  // dchi/dR (3 x the padded tables), the boxes' replicas' offsets in them, and
+  // dL/dR [n_atm][3]
+  const double *gmu;
+  double *vjp;
+  size_t vjp_stride;  // doubles per CTA
+  double *g_veff;
+  int gex;
+  const double *dtab;
+  long long dtab_stride;
+  const long long *rep_off;
+  double *g_atoms;
   unsigned long long *proj_points;  // [3]: ball points x steps (all, Chebyshev only), ball-in-window points x steps
 };
 
@@ -185,6 +199,10 @@ cudaError_t launch_sweep(const SweepArgs &a, int grid, cudaStream_t s);
 // storage of the Chebyshev vectors (the FP32-mixed form), else FP64.
 cudaError_t sweep_forces_per_sm(const SweepArgs &a, int single, int *per_sm);
 cudaError_t launch_sweep_forces(const SweepArgs &a, int single, int grid, cudaStream_t s);
+// Adjoint on the sweep kernel (sqb_sweep_vjp.cu); doubles of scratch per CTA.
+size_t sweep_vjp_doubles(int n, int npl);
+cudaError_t sweep_vjp_per_sm(const SweepArgs &a, int *per_sm);
+cudaError_t launch_sweep_vjp(const SweepArgs &a, int grid, cudaStream_t s);
 // Layered fields from the padded projector tables: ids and values of every
 // replica's ball on the extended grid (ex x ey x ez points, rows of pitch
 // values; fields zeroed / set empty first).

@@ -84,6 +84,7 @@ struct Shared {
   short e_pb[MAXE];  // first local projector instance
   int e_gpb[MAXE];   // first global projector id
   int e_atom[MAXE];  // global atom (force passes)
+  int e_r[MAXE];     // index of the replica's box
   // local projector instances p < n_pi
   short pi_e[MAXP];
   int pi_g[MAXP];
@@ -911,6 +912,7 @@ static __device__ void setup_node(const SweepArgs &a, Shared &S) {
         S.e_np[pos] = (unsigned char)((b.w >> 8) & 0xff);
         S.e_t[pos] = (unsigned char)((b.w >> 16) & 0xff);
         S.e_gpb[pos] = a.rep_gpb[r];
+        S.e_r[pos] = r;
         S.e_atom[pos] = a.rep_atom ? a.rep_atom[r] : -1;
       } else {
         atomicOr(a.status, ST_CAPACITY);

@@ -1,5 +1,5 @@
-"""The sweep kernel's tiles and layers against the plane-streaming kernel, at the sizes
-where they can go wrong.
+"""The sweep kernel's tiles, layers and adjoint against the plane-streaming kernel, at the
+sizes where they can go wrong.
 
 The window edges are the smallest and largest of every tile (pairs of columns: windows
 that start at odd and even columns of the halo'd block, the last pair half outside), for
@@ -57,6 +57,15 @@ def test_tiles_match_plane_kernel(system, nloc):
     for form in (0, 1):
         a, b = _both(_params("forces", system, nloc, form, per_cell=20 if system == "lih" or nloc > 13 else 12))
         assert _rel(a, b) <= (1e-5 if form else 1e-11), form
+
+
+@pytest.mark.parametrize("system,nloc,npl", [("al", 4, 4), ("al", 9, 16), ("al", 10, 20), ("al", 15, 36),
+                                             ("al", 17, 12), ("lih", 8, 20), ("lih", 16, 64), ("lih", 19, 16)])
+def test_adjoint_matches_plane_kernel(system, nloc, npl):
+    """Block remainders of the quadratic form (16 vectors, 8 at a time), one block and several."""
+    (gv, ga), (gv0, ga0) = _both(_params("vjp", system, nloc, npl=npl, per_cell=20))
+    assert _rel(gv, gv0) <= 1e-12
+    assert _rel(ga, ga0) <= 1e-11
 
 
 def test_layers_of_displaced_lih_fit():
