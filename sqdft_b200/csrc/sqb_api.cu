@@ -117,6 +117,8 @@ struct sqb_ctx {
   int *d_loc_type = nullptr, *d_loc_atom = nullptr, *d_loc_box = nullptr, *d_loc_size = nullptr;
   long long *d_loc_off = nullptr, *d_loc_scr_off = nullptr;
   double *d_loc_xyz = nullptr, *d_loc_tab = nullptr, *d_loc_Z = nullptr;
+  double4 *d_loc_coef = nullptr;  // interval cubics and radius bins of the tables
+  int *d_loc_bin = nullptr;
   double *d_loc_fields = nullptr;  // b, b_tilda, Vc, rho_at, phi (+halo), partial sums
   size_t loc_fields_bytes = 0;
   double *d_loc_scr = nullptr;     // ForcesLocal scratch boxes and per-CTA force sums
@@ -831,7 +833,7 @@ int sqb_destroy(sqb_ctx *c) {
                   c->d_lmax, c->d_xk, c->d_ctab, c->d_partial, c->d_result, c->d_rho, c->d_ci, c->d_fslots,
                   c->d_f, c->d_tmp, c->d_sens, c->d_loss, c->d_fermi, c->d_loc_type, c->d_loc_atom,
                   c->d_loc_box, c->d_loc_size, c->d_loc_off, c->d_loc_scr_off, c->d_loc_xyz, c->d_loc_tab,
-                  c->d_loc_Z, c->d_loc_fields, c->d_loc_scr};
+                  c->d_loc_Z, c->d_loc_coef, c->d_loc_bin, c->d_loc_fields, c->d_loc_scr};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   drop_graph(c);
@@ -2199,6 +2201,8 @@ LocalArgs local_args(const sqb_ctx *c) {
   a.rep_xyz = c->d_loc_xyz;
   a.rep_box = c->d_loc_box;
   a.tab = c->d_loc_tab;
+  a.coef = c->d_loc_coef;
+  a.bin = c->d_loc_bin;
   a.typ_off = c->d_loc_off;
   a.typ_size = c->d_loc_size;
   a.Z = c->d_loc_Z;
@@ -2283,6 +2287,11 @@ int sqb_set_local_atoms(sqb_ctx *c, int n_typ, const sqb_local_species *types, i
   CK(cudaMemcpy(c->d_loc_off, off.data(), n_typ * sizeof(long long), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_loc_size, size.data(), n_typ * sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_loc_Z, Z.data(), n_typ * sizeof(double), cudaMemcpyHostToDevice));
+  CK(dalloc(&c->d_loc_coef, local_coef_count(total)));
+  CK(dalloc(&c->d_loc_bin, local_bin_count(n_typ)));
+  CK(cudaStreamSynchronize(cudaStreamLegacy));  // the copies above
+  CK(launch_local_prepare(n_typ, c->d_loc_tab, c->d_loc_off, c->d_loc_size, c->d_loc_coef, c->d_loc_bin, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   if (n_rep > 0) {
     CK(cudaMemcpy(c->d_loc_type, rep_type, n_rep * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c->d_loc_atom, rep_atom, n_rep * sizeof(int), cudaMemcpyHostToDevice));

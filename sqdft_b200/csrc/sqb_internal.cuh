@@ -316,6 +316,8 @@ struct LocalArgs {
   const double *rep_xyz;  // [n_rep][3]
   const int *rep_box;     // [n_rep][6]: xstart, xend, ystart, yend, zstart, zend (global nodes)
   const double *tab;      // per type [5][size]: grid, rVloc, DVloc, uu, Duu
+  const double4 *coef;    // per type [2][size]: cubics of rVloc and uu (launch_local_prepare)
+  const int *bin;         // per type: grid points at the radius bins' edges
   const long long *typ_off;
   const int *typ_size;
   const double *Z;
@@ -333,6 +335,11 @@ struct LocalArgs {
   const long long *scr_off;
   double *fpart;
 };
+// The types' interval cubics and radius bins from their tables; their sizes.
+size_t local_coef_count(long long table_values);
+size_t local_bin_count(int n_typ);
+cudaError_t launch_local_prepare(int n_typ, const double *tab, const long long *off, const int *size, double4 *coef,
+                                 int *bin, cudaStream_t s);
 // Tile edge of the charge-density kernel and its CTA count for the block.
 constexpr int LOC_TILE = 8;
 int charge_density_ctas(const int np[3]);

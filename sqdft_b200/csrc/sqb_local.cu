@@ -5,7 +5,9 @@
 // intersection box, b_J = -(1/4 pi) Lap_h V_J and the same of the smooth
 // reference potential V~_J, with V_J the spline of r Vloc over r.
 //
-// Charge density: one CTA per 8^3 tile of the block, one thread per node.
+// Charge density: one CTA per 8^3 tile of the block, two threads per node (one
+// for V_J, one for V~_J: the tile's 128 KB of shared memory leave room for one
+// CTA per SM, and its 32 warps hide the lookups' latency where 16 did not).
 // The CTA lists the replicas that meet its tile, in the reference's loop
 // order, and for each one puts V_J and V~_J on the tile and its FDN halo
 // into shared memory. Each thread then adds the replica's terms to its own
@@ -31,29 +33,71 @@ constexpr int LLIST = 512;        // replicas tested per list pass (one per thre
 constexpr double PI = 3.14159265358979323846;  // M_PI
 constexpr double TOL = 1e-12;                  // TEMP_TOL of the reference
 
-// ispline_gen (spline.cpp:11-55) at one point: the first grid point >= x,
-// stepped back unless equal; false out of the table's range.
-__device__ bool spline_at(const double *X, const double *Y, const double *YD, int len, double x, double &out) {
-  if (!(x >= X[0] && x <= X[len - 1])) return false;
-  int lo = 0, hi = len - 1;
+// A type's prepared radial tables (launch_local_prepare): per interval the
+// cubic's coefficients of rVloc and of the atomic density, as ispline_gen
+// forms them at each point, and per bin of the radius the first grid point at
+// or above the bin's lower edge.  A bin is the exponent and the top six
+// mantissa bits of the radius (1/64 of an octave), so a lookup searches the one
+// or two grid points of its bin and not the whole grid: three dependent loads
+// in place of the binary search's eleven and no division.
+constexpr int BIN0 = (1023 - 12) << 6;  // bins start at 2^-12 and end at 2^9
+constexpr int NBIN = 21 << 6;
+__device__ __forceinline__ int radius_bin(double x) {
+  const int b = (__double2hiint(x) >> 14) - BIN0;
+  return b < 0 ? 0 : (b >= NBIN ? NBIN - 1 : b);
+}
+
+// First grid point >= x among [lo, hi].
+__device__ __forceinline__ int first_at_or_above(const double *X, int lo, int hi, double x) {
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
     if (X[mid] < x) lo = mid + 1;
     else hi = mid;
   }
-  int j = lo;
+  return lo;
+}
+
+__global__ void local_prepare_kernel(const double *tab, const long long *off, const int *size, double4 *coef, int *bin) {
+  const int t = blockIdx.y, len = size[t];
+  const double *X = tab + off[t];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * len + NBIN + 1; i += gridDim.x * blockDim.x) {
+    if (i < 2 * len) {
+      const int f = i >= len, j = i - f * len;
+      if (j > len - 2) continue;
+      const double *Y = X + (f ? 3 : 1) * (size_t)len, *YD = Y + len;
+      const double dx = 1.0 / (X[j + 1] - X[j]);
+      const double dy = (Y[j + 1] - Y[j]) * dx;
+      const double A2 = dx * (3.0 * dy - 2.0 * YD[j] - YD[j + 1]);
+      const double A3 = dx * dx * (-2.0 * dy + YD[j] + YD[j + 1]);
+      coef[2 * (off[t] / 5) + i] = make_double4(Y[j], YD[j], A2, A3);
+    } else {
+      const int k = i - 2 * len;
+      const double edge = __hiloint2double((k + BIN0) << 14, 0);
+      bin[t * (NBIN + 1) + k] = k == 0 ? 0 : (k == NBIN ? len - 1 : first_at_or_above(X, 0, len - 1, edge));
+    }
+  }
+}
+
+// ispline_gen (spline.cpp:11-55) at one point: the interval below the first
+// grid point >= x, stepped back unless equal (false out of the table's range),
+// and the cubic of field f (0 rVloc, 1 the atomic density) there.
+__device__ __forceinline__ bool spline_interval(const LocalArgs &a, int t, double x, int &j) {
+  const double *X = a.tab + a.typ_off[t];
+  const int len = a.typ_size[t];
+  if (!(x >= X[0] && x <= X[len - 1])) return false;
+  const int *bin = a.bin + t * (NBIN + 1) + radius_bin(x);
+  j = first_at_or_above(X, bin[0], bin[1], x);
   if (x < X[j]) j--;
   if (j > len - 2) j = len - 2;
   if (j < 0) j = 0;
-  const double p1 = X[j];
-  const double dx = 1.0 / (X[j + 1] - X[j]);
-  const double dy = (Y[j + 1] - Y[j]) * dx;
-  const double A0 = Y[j], A1 = YD[j];
-  const double A2 = dx * (3.0 * dy - 2.0 * YD[j] - YD[j + 1]);
-  const double A3 = dx * dx * (-2.0 * dy + YD[j] + YD[j + 1]);
-  const double t = x - p1;
-  out = ((A3 * t + A2) * t + A1) * t + A0;
   return true;
+}
+__device__ __forceinline__ double spline_value(const LocalArgs &a, int t, int f, int j, double x) {
+  const double *X = a.tab + a.typ_off[t];
+  const double2 *c = reinterpret_cast<const double2 *>(a.coef + 2 * (a.typ_off[t] / 5) + (size_t)f * a.typ_size[t] + j);
+  const double2 lo = c[0], hi = c[1];
+  const double u = x - X[j];
+  return ((hi.y * u + hi.x) * u + lo.y) * u + lo.x;
 }
 
 // Distance of global node (gi, gj, gk) from a replica (initialize.cpp:571).
@@ -65,12 +109,15 @@ __device__ __forceinline__ double node_radius(const LocalArgs &a, const double *
 // VlocJ and VlocJ_tilda of a replica of type t at distance r
 // (initialize.cpp:573-597, forces.cpp:126-143).
 __device__ bool vloc_pair(const LocalArgs &a, int t, double r, double &v, double &vt) {
-  const double *G = a.tab + a.typ_off[t];
-  const int len = a.typ_size[t];
-  const double *rV = G + len, *DV = G + 2 * (size_t)len;
-  double s;
-  if (!spline_at(G, rV, DV, len, r, s)) return false;
-  v = fabs(r - 0.0) < TOL ? rV[1] / G[1] : s / r;
+  int j;
+  if (!spline_interval(a, t, r, j)) return false;
+  const double s = spline_value(a, t, 0, j, r);
+  if (fabs(r - 0.0) < TOL) {
+    const double *G = a.tab + a.typ_off[t];
+    v = G[a.typ_size[t] + 1] / G[1];
+  } else {
+    v = s / r;
+  }
   const double rc = a.rc_tilda, Z = a.Z[t];
   if (r < rc)
     vt = -Z * (9 * pow(r, 7) - 30 * rc * pow(r, 6) + 28 * rc * rc * pow(r, 5) - 14 * pow(rc, 5) * pow(r, 2) +
@@ -104,17 +151,18 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
   return s;  // valid in thread 0
 }
 
-__global__ void __launch_bounds__(LT *LT *LT) charge_density_kernel(LocalArgs a) {
+__global__ void __launch_bounds__(2 * LT *LT *LT) charge_density_kernel(LocalArgs a) {
   extern __shared__ double sm[];
   double *sV = sm, *sVt = sm + LH3;
   __shared__ int list[LLIST];
-  __shared__ int wcount[LT * LT * LT / 32 + 1];
+  __shared__ int wcount[2 * LT * LT * LT / 32 + 1];
   __shared__ int nlist;
   __shared__ double red[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
   const int NX = a.np[0], NY = a.np[1], NZ = a.np[2];
   const int x0 = blockIdx.x * LT, y0 = blockIdx.y * LT, z0 = blockIdx.z * LT;  // tile origin (block nodes)
-  const int li = tid % LT, lj = (tid / LT) % LT, lk = tid / (LT * LT);
+  const int half = tid / (LT * LT * LT);  // 0: V_J and the atomic density, 1: V~_J and Vc
+  const int li = tid % LT, lj = (tid / LT) % LT, lk = tid / (LT * LT) % LT;
   const int x = x0 + li, y = y0 + lj, z = z0 + lk;
   const bool in = x < NX && y < NY && z < NZ;
   const int gx = x + a.pnode_s[0], gy = y + a.pnode_s[1], gz = z + a.pnode_s[2];
@@ -123,8 +171,8 @@ __global__ void __launch_bounds__(LT *LT *LT) charge_density_kernel(LocalArgs a)
   const int tx1 = min(x0 + LT, NX) - 1 + a.pnode_s[0], ty1 = min(y0 + LT, NY) - 1 + a.pnode_s[1],
             tz1 = min(z0 + LT, NZ) - 1 + a.pnode_s[2];
   const double h = a.delta;
-  double b = 0.0, bt = 0.0, vc = 0.0, ra = 0.0;
-  double eS = 0.0, nC = 0.0, nE = 0.0, nCt = 0.0, eSt = 0.0;
+  double b = 0.0, vc = 0.0, ra = 0.0;       // b of the thread's field; Vc (half 1), rho_at (half 0)
+  double eS = 0.0, nC = 0.0, nE = 0.0;
   for (int base = 0; base < a.n_rep; base += LLIST) {
     // the replicas of [base, base + LLIST) whose box meets the tile, in order
     const int r = base + tid;
@@ -171,37 +219,39 @@ __global__ void __launch_bounds__(LT *LT *LT) charge_density_kernel(LocalArgs a)
       if (in && gx >= bx[0] && gx <= bx[1] && gy >= bx[2] && gy <= bx[3] && gz >= bx[4] && gz <= bx[5]) {
         const long long hc = ((long long)(lk + FDN) * LH + (lj + FDN)) * LH + (li + FDN);
         // initialize.cpp:583-588: the atomic density at the node
-        const double *G = a.tab + a.typ_off[t];
-        const int len = a.typ_size[t];
-        double rho_temp;
-        if (!spline_at(G, G + 3 * (size_t)len, G + 4 * (size_t)len, len, node_radius(a, c, gx, gy, gz), rho_temp)) {
-          atomicOr(a.status, ST_SPLINE_RANGE);
-          rho_temp = 0.0;
+        if (!half) {
+          const double r = node_radius(a, c, gx, gy, gz);
+          double rho_temp = 0.0;
+          int j;
+          if (spline_interval(a, t, r, j)) rho_temp = spline_value(a, t, 1, j, r);
+          else atomicOr(a.status, ST_SPLINE_RANGE);
+          ra += rho_temp;
+          nE += rho_temp * h * h * h;
         }
-        ra += rho_temp;
-        nE += rho_temp * h * h * h;
         // initialize.cpp:600-626
-        const double bJ = neg_lap(a, sV, hc, LH, LH * LH), bJt = neg_lap(a, sVt, hc, LH, LH * LH);
+        const double *f = half ? sVt : sV;
+        const double bJ = neg_lap(a, f, hc, LH, LH * LH);
         b += bJ;
-        eS += 0.5 * bJ * sV[hc] * h * h * h;
+        eS += 0.5 * bJ * f[hc] * h * h * h;
         nC += bJ * h * h * h;
-        bt += bJt;
-        eSt += 0.5 * bJt * sVt[hc] * h * h * h;
-        nCt += bJt * h * h * h;
-        vc += sVt[hc] - sV[hc];
+        if (half) vc += sVt[hc] - sV[hc];
       }
       __syncthreads();
     }
   }
   if (in) {
     const long long g = ((long long)z * NY + y) * NX + x;
-    a.b[g] = b;
-    a.b_tilda[g] = bt;
-    a.vc[g] = vc;
-    a.rho_at[g] = ra;
+    if (half) {
+      a.b_tilda[g] = b;
+      a.vc[g] = vc;
+    } else {
+      a.b[g] = b;
+      a.rho_at[g] = ra;
+    }
   }
   const int nb = gridDim.x * gridDim.y * gridDim.z, blk = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  const double sums[5] = {eS, nC, nE, nCt, eSt};
+  // (the other half's zeros leave each sum as it is)
+  const double sums[5] = {half ? 0.0 : eS, half ? 0.0 : nC, nE, half ? nC : 0.0, half ? eS : 0.0};
   for (int k = 0; k < 5; k++) {
     const double s = block_sum(sums[k], red);
     if (tid == 0) a.partial[k * nb + blk] = s;
@@ -323,6 +373,15 @@ __global__ void local_force_kernel(LocalArgs a, int r0) {
 
 }  // namespace
 
+size_t local_coef_count(long long table_values) { return (size_t)(2 * (table_values / 5)); }
+size_t local_bin_count(int n_typ) { return (size_t)n_typ * (NBIN + 1); }
+
+cudaError_t launch_local_prepare(int n_typ, const double *tab, const long long *off, const int *size, double4 *coef,
+                                 int *bin, cudaStream_t s) {
+  local_prepare_kernel<<<dim3(16, n_typ), 256, 0, s>>>(tab, off, size, coef, bin);
+  return cudaGetLastError();
+}
+
 int charge_density_ctas(const int np[3]) {
   return ((np[0] + LT - 1) / LT) * ((np[1] + LT - 1) / LT) * ((np[2] + LT - 1) / LT);
 }
@@ -332,7 +391,7 @@ cudaError_t launch_charge_density(const LocalArgs &a, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(charge_density_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const dim3 grid((a.np[0] + LT - 1) / LT, (a.np[1] + LT - 1) / LT, (a.np[2] + LT - 1) / LT);
-  charge_density_kernel<<<grid, LT * LT * LT, smem, s>>>(a);
+  charge_density_kernel<<<grid, 2 * LT * LT * LT, smem, s>>>(a);
   return cudaGetLastError();
 }
 

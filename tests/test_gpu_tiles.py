@@ -1,5 +1,6 @@
-"""The sweep kernel's tiles, layers and adjoint against the plane-streaming kernel, at the
-sizes where they can go wrong.
+"""The sweep kernel's tiles, layers and adjoint against the plane-streaming kernel, and
+the radial lookups of the pseudocharge kernels against the oracle, at the sizes where
+they can go wrong.
 
 The window edges are the smallest and largest of every tile (pairs of columns: windows
 that start at odd and even columns of the halo'd block, the last pair half outside), for
@@ -82,3 +83,25 @@ def test_layers_of_displaced_lih_fit():
             ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
             b = cases.run(s)
         assert _rel(a["rho_pj"], b["rho_pj"]) <= 3e-7
+
+
+@pytest.mark.parametrize("grid_kind", ["uniform", "coarse", "octaves"])
+def test_radial_lookup_on_other_grids(grid_kind):
+    """Radial grids with many points per lookup bin, with many bins per point, and with
+    points on the bins' edges: b and rho_at equal the oracle's bit for bit."""
+    from oracle.pyoracle import LocalOracle
+    from perf import cases
+    from sqdft_b200 import sq
+
+    p = dict(kind="local", system="al", form=0, cells=1, per_cell=10, block="9x8x10", nloc=1, npl=4, kt=10.0)
+    grid, loc, _ = cases._local_inputs(p, 5)
+    r = {"uniform": np.linspace(0.0, 40.0, 6001), "coarse": np.linspace(0.0, 40.0, 41),
+         "octaves": np.concatenate([[0.0], 2.0 ** (np.arange(-14 * 8, 6 * 8) / 8)])}[grid_kind]
+    a = 1.1
+    uu = np.exp(-(r / a) ** 2)
+    loc.tables = [np.stack([r, -3 * np.tanh(r), -3 / np.cosh(r) ** 2, uu, -2 * r / a ** 2 * uu]) for _ in loc.tables]
+    with sq.LocalContext(grid, loc) as ctx:
+        out = ctx.charge_density()
+    ref = LocalOracle(grid, loc).charge_density()
+    assert np.array_equal(out["b"], ref["b"])
+    assert np.array_equal(out["rho_at"], ref["rho_at"])
