@@ -1703,7 +1703,7 @@ int sqb_autotune_sweep(sqb_ctx *c, int sample, int *rows, double *ms_out) {
   int best = 0;
   for (int k = 0; k < 2; k++) {
     c->sweep_ry = 2 + k;
-    if (sweep_rows(c) != c->sweep_ry) continue;  // not covered for this window
+    if (c->sweep_ry == 3 && sweep_rows(c) != 3) continue;  // not covered for this window
     NodeArgs a;
     fill_node_args(c, a);
     a.mode = MODE_SQ;
