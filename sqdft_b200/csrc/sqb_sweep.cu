@@ -79,7 +79,12 @@ namespace sweep {
 cudaError_t tile_setup(const void *kernel, const SweepArgs &a, int *per_sm) {
   if (kernel == nullptr || a.n > MAXN || sweep_threads_of(a.n, a.ry) != a.nsweep) return cudaErrorInvalidConfiguration;
   const size_t smem = sweep_smem(a.n, a.pmax, a.n_gproj, a.ry);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the device's limit, not this launch's size: contexts of other windows on
+  // other threads share the kernel's attribute
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
   if (e == cudaSuccess && per_sm) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, a.nsweep, smem);
     if (e == cudaSuccess && *per_sm < 1) e = cudaErrorInvalidConfiguration;
