@@ -3,7 +3,7 @@
 // Chebyshev moments, ClenshawCurtisSpectralQuadrature sq.cpp:530-661) on
 // sm_100a, built around a branch-free nonlocal term.
 //
-// One persistent CTA per SM takes grid nodes from an atomic queue.  Every
+// Persistent CTAs, as many as fit on an SM, take grid nodes from an atomic queue.  Every
 // matvec H v = -1/2 Lap_h v + Veff v + Vnl v on a node's (2nloc+1)^3 window
 // (HsubTimesVec sq.cpp:838-929, VnlocsubTimesVec nonlocal.cpp:20-215; v zero
 // outside the window) is one sweep over the window's z-planes:
