@@ -73,6 +73,7 @@ struct sqb_ctx {
   int node_kernel = SQB_KERNEL_AUTO;
   int sweep_ry = 0;  // window rows per sweep-kernel thread (0: automatic)
   int lay_state = 0;  // 0 not built, 1 built and usable, -1 the sweep kernel does not cover this context
+  bool lay_first_fit = false;  // the layers are those of first fit in replica order
   int n_gproj = 0, lay_pmax = 1, n_lrep = 0;
   unsigned long long *d_lay_id = nullptr;
   double *d_lay_chi = nullptr;
@@ -337,7 +338,8 @@ int ensure_layers(sqb_ctx *c) {
   };
   int n_layers = 0;
   for (int i = 0; i < nb; i++) n_layers = std::max(n_layers, (layer_of[i] = first_free(i)) + 1);
-  if (n_layers > LAYERS) {
+  const bool first_fit = n_layers <= LAYERS;
+  if (!first_fit) {
     // First fit in replica order can start two far-apart balls on layers that
     // their common neighbours then cannot share.  Colouring next the ball whose
     // neighbours already use the most layers (DSATUR, Brelaz 1979) finds the
@@ -383,6 +385,7 @@ int ensure_layers(sqb_ctx *c) {
                       sweep_rows_supported(c->n, 1) && sweep_smem(c->n, pm, ngp, 1) <= (size_t)optin &&
                       c->n_typ < 256;
   if (!usable) return SQB_OK;
+  c->lay_first_fit = first_fit;
   c->n_gproj = ngp;
   c->lay_pmax = pm;
   c->n_lrep = (int)boxes.size();
@@ -416,7 +419,7 @@ int ensure_layers(sqb_ctx *c) {
   return SQB_OK;
 }
 
-// Whether the SQ node work of this context runs on the sweep kernel.
+// Whether the nonlocal forces of this context run on the sweep kernel.
 int use_sweep(sqb_ctx *c, bool *yes) {
   *yes = false;
   if (c->node_kernel == SQB_KERNEL_PLANE) return SQB_OK;
@@ -424,6 +427,27 @@ int use_sweep(sqb_ctx *c, bool *yes) {
   if (rc) return rc;
   if (c->lay_state != 1) return c->node_kernel == SQB_KERNEL_SWEEP ? SQB_ERR_UNSUPPORTED : SQB_OK;
   *yes = true;
+  return SQB_OK;
+}
+
+// Kernel of the SQ node work: the plane-streaming kernel, the sweep kernel, or
+// its one-column tile.  The sweep kernel runs wherever it covers the context
+// but for the FP64 form with several projectors per slot, whose long Lanczos
+// runs end at a bound that follows the order of the sums (sqb_sweep_cols.cu):
+// that form keeps the kernel its results have always come from, the one-column
+// tile under first-fit layers and else the plane-streaming kernel, unless
+// SQB_KERNEL_SWEEP is asked for.
+enum class SqKernel { Plane, Sweep, Columns };
+int sq_kernel(sqb_ctx *c, bool fp64, SqKernel *k) {
+  bool sw = false;
+  const int rc = use_sweep(c, &sw);
+  if (rc) return rc;
+  *k = sw ? SqKernel::Sweep : SqKernel::Plane;
+  if (!sw || !fp64 || c->lay_pmax == 1) return SQB_OK;
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+  if (c->lay_first_fit && sweep_cols_supported(c->n, c->n_gproj, 2, (size_t)optin)) *k = SqKernel::Columns;
+  else if (c->node_kernel != SQB_KERNEL_SWEEP) *k = SqKernel::Plane;
   return SQB_OK;
 }
 
@@ -496,12 +520,26 @@ int sweep_grid(sqb_ctx *c, int per_sm, SweepArgs &s, int *grid) {
   return rc;
 }
 
-// Arguments, grid and scratch of an SQ launch on the sweep kernel.
-int prepare_sq_sweep(sqb_ctx *c, const NodeArgs &a, const int *d_list, int count, SweepArgs &s, int *grid) {
+// Window rows per thread of the one-column tile: three where asked for and covered, else two.
+int column_rows(const sqb_ctx *c) {
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+  return c->sweep_ry == 3 && sweep_cols_supported(c->n, c->n_gproj, 3, (size_t)optin) ? 3 : 2;
+}
+
+// Arguments, grid and scratch of an SQ launch on the sweep kernel (cols: its
+// one-column tile).
+int prepare_sq_sweep(sqb_ctx *c, const NodeArgs &a, bool cols, const int *d_list, int count, SweepArgs &s, int *grid) {
   fill_sweep_args(c, d_list, count, s);
   s.form = a.lq ? 2 : (a.mixed ? 1 : 0);
   int per_sm = 0;
-  CK(sweep_per_sm(s, &per_sm));
+  if (cols) {
+    s.ry = column_rows(c);
+    s.nsweep = sweep_cols_threads(c->n, s.ry);
+    CK(sweep_cols_per_sm(s, &per_sm));
+  } else {
+    CK(sweep_per_sm(s, &per_sm));
+  }
   return sweep_grid(c, per_sm, s, grid);
 }
 
@@ -509,14 +547,14 @@ int prepare_sq_sweep(sqb_ctx *c, const NodeArgs &a, const int *d_list, int count
 // with the outputs of `a`, on the sweep kernel where it covers the context,
 // else on the plane-streaming node kernel.
 int run_sq_nodes(sqb_ctx *c, NodeArgs &a, const int *d_list, int count) {
-  bool sw = false;
-  int rc = use_sweep(c, &sw);
+  SqKernel k{};
+  int rc = sq_kernel(c, !a.mixed && !a.lq, &k);
   if (rc) return rc;
-  c->stats.node_kernel = sw ? SQB_KERNEL_SWEEP : SQB_KERNEL_PLANE;
-  if (!sw) return run_nodes(c, a, d_list, count);
+  c->stats.node_kernel = k == SqKernel::Plane ? SQB_KERNEL_PLANE : SQB_KERNEL_SWEEP;
+  if (k == SqKernel::Plane) return run_nodes(c, a, d_list, count);
   SweepArgs s;
   int grid = 0;
-  rc = prepare_sq_sweep(c, a, d_list, count, s, &grid);
+  rc = prepare_sq_sweep(c, a, k == SqKernel::Columns, d_list, count, s, &grid);
   if (rc) return rc;
   s.lanczos_tol = a.lanczos_tol;
   s.lz_chk = a.lz_chk;
@@ -529,7 +567,7 @@ int run_sq_nodes(sqb_ctx *c, NodeArgs &a, const int *d_list, int count) {
   CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->d_proj_points, 0, 3 * sizeof(unsigned long long), c->stream));
-  CK(launch_sweep(s, grid, c->stream));
+  CK(k == SqKernel::Columns ? launch_sweep_cols(s, grid, c->stream) : launch_sweep(s, grid, c->stream));
   return SQB_OK;
 }
 
@@ -1434,9 +1472,11 @@ static int build_step_graph(sqb_ctx *c) {
   a.lmax = c->d_lmax;
   a.lanczos_iters = c->d_iters;
   {  // allocate what the captured launches use (no allocation inside a capture)
+    SqKernel k{};
     SweepArgs s;
     int grid = 0;
-    const int rc0 = prepare_sq_sweep(c, a, c->d_nodes, c->nnode, s, &grid);
+    int rc0 = sq_kernel(c, !a.mixed && !a.lq, &k);
+    if (!rc0) rc0 = prepare_sq_sweep(c, a, k == SqKernel::Columns, c->d_nodes, c->nnode, s, &grid);
     if (rc0) return rc0;
   }
   FermiArgs fa = fermi_args(c);
@@ -1562,10 +1602,10 @@ static int spectral_quadrature(sqb_ctx *c, int scf_iter, double *lambda_f, doubl
   const double tol_eff = std::max(c->g.lanczos_tol, c->mixed_lanczos_tol);
   const bool defect = c->precision != SQB_FP64 && c->defect_budget > 0.0 && tol_eff > c->g.lanczos_tol;
   if (c->use_graph == 2 && !c->allreduce && !defect && c->have_veff && c->have_atoms && c->have_proj) {
-    bool sw = false;
-    int rc0 = use_sweep(c, &sw);
+    SqKernel k{};
+    int rc0 = sq_kernel(c, c->precision == SQB_FP64, &k);
     if (rc0) return rc0;
-    if (sw) return run_step_graph(c, scf_iter, *lambda_f, lambda_f, rho, rho_pj, ci, chi, zee, ebs, eent);
+    if (k != SqKernel::Plane) return run_step_graph(c, scf_iter, *lambda_f, lambda_f, rho, rho_pj, ci, chi, zee, ebs, eent);
   }
   int rc = sqb_lanczos_moments(c, chi, zee, rho_pj, nullptr, nullptr, nullptr);
   if (rc) return rc;
@@ -1685,10 +1725,10 @@ int sqb_autotune_sweep(sqb_ctx *c, int sample, int *rows, double *ms_out) {
   if (!c || sample < 0) return SQB_ERR_ARG;
   if (!c->have_veff || !c->have_atoms || !c->have_proj) return SQB_ERR_STATE;
   cudaSetDevice(c->device);
-  bool sw = false;
-  int rc = use_sweep(c, &sw);
+  SqKernel kernel{};
+  int rc = sq_kernel(c, c->precision == SQB_FP64, &kernel);
   if (rc) return rc;
-  if (!sw) return SQB_ERR_UNSUPPORTED;
+  if (kernel == SqKernel::Plane) return SQB_ERR_UNSUPPORTED;
   const int N = c->nnode;
   int count = sample > 0 ? sample : 2 * c->sms;
   if (count > N) count = N;
@@ -1703,7 +1743,8 @@ int sqb_autotune_sweep(sqb_ctx *c, int sample, int *rows, double *ms_out) {
   int best = 0;
   for (int k = 0; k < 2; k++) {
     c->sweep_ry = 2 + k;
-    if (c->sweep_ry == 3 && sweep_rows(c) != 3) continue;  // not covered for this window
+    if (c->sweep_ry == 3 && (kernel == SqKernel::Columns ? column_rows(c) : sweep_rows(c)) != 3)
+      continue;  // not covered for this window
     NodeArgs a;
     fill_node_args(c, a);
     a.mode = MODE_SQ;

@@ -160,7 +160,7 @@ struct SweepArgs {
   unsigned char *scratch;
   size_t scratch_stride;  // bytes per CTA: three window vectors (FP64), then the flush buffer
   int nsweep;             // threads of the block (a multiple of 32)
-  int ry;                 // window rows per thread (1, or 3 up to 33-wide windows)
+  int ry;                 // window rows per thread (1, or 3 up to 33-wide windows; one column per thread: 2 or 3)
   double *chi, *zee, *rho_pj, *lmin, *lmax;
   int *lanczos_iters;
   // ForcesNonLocal (sweep_force_kernel): bounds in chi, zee (inputs), the
@@ -195,6 +195,12 @@ bool sweep_rows_supported(int n, int ry);
 size_t sweep_scratch_bytes(int n, int pmax);  // scratch per CTA
 cudaError_t sweep_per_sm(const SweepArgs &a, int *per_sm);  // resident CTAs per SM of the launch's kernel
 cudaError_t launch_sweep(const SweepArgs &a, int grid, cudaStream_t s);
+// The FP64 SQ step of three projectors per slot with one column per thread
+// (sqb_sweep_cols.cu); ry: window rows per thread, 2 or 3.
+bool sweep_cols_supported(int n, int n_gproj, int ry, size_t smem_limit);
+int sweep_cols_threads(int n, int ry);
+cudaError_t sweep_cols_per_sm(const SweepArgs &a, int *per_sm);
+cudaError_t launch_sweep_cols(const SweepArgs &a, int grid, cudaStream_t s);
 // ForcesNonLocal on the sweep kernel (sqb_sweep_forces.cu); single: FP32
 // storage of the Chebyshev vectors (the FP32-mixed form), else FP64.
 cudaError_t sweep_forces_per_sm(const SweepArgs &a, int single, int *per_sm);

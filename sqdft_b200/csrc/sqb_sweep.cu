@@ -76,9 +76,8 @@ size_t sweep_scratch_bytes(int n, int pmax) {
 
 namespace sweep {
 
-cudaError_t tile_setup(const void *kernel, const SweepArgs &a, int *per_sm) {
-  if (kernel == nullptr || a.n > MAXN || sweep_threads_of(a.n, a.ry) != a.nsweep) return cudaErrorInvalidConfiguration;
-  const size_t smem = sweep_smem(a.n, a.pmax, a.n_gproj, a.ry);
+cudaError_t kernel_setup(const void *kernel, int threads, size_t smem, int *per_sm) {
+  if (kernel == nullptr) return cudaErrorInvalidConfiguration;
   // the device's limit, not this launch's size: contexts of other windows on
   // other threads share the kernel's attribute
   int dev = 0, optin = 0;
@@ -86,10 +85,15 @@ cudaError_t tile_setup(const void *kernel, const SweepArgs &a, int *per_sm) {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
   if (e == cudaSuccess && per_sm) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, a.nsweep, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem);
     if (e == cudaSuccess && *per_sm < 1) e = cudaErrorInvalidConfiguration;
   }
   return e;
+}
+
+cudaError_t tile_setup(const void *kernel, const SweepArgs &a, int *per_sm) {
+  if (a.n > MAXN || sweep_threads_of(a.n, a.ry) != a.nsweep) return cudaErrorInvalidConfiguration;
+  return kernel_setup(kernel, a.nsweep, sweep_smem(a.n, a.pmax, a.n_gproj, a.ry), per_sm);
 }
 
 }  // namespace sweep

@@ -986,19 +986,33 @@ static __device__ void count_proj_points(const SweepArgs &a, Shared &S, long lon
   atomicAdd(a.proj_points + 2, win * (unsigned long long)steps);
 }
 
+// What lanczos and moments need of a kernel's tile: its sweep and the layout of
+// its window vectors (rows of `cols` values, window column x at x + shift).
+template <int PM_, int RY, int NT>
+struct PairTile {
+  static constexpr int PM = PM_;
+  static __device__ __forceinline__ int cols(int n) { return pair_cols(n); }
+  static __device__ __forceinline__ int shift(const Shared &S) { return S.gi & 1; }
+  template <typename T, int SK>
+  static __device__ __forceinline__ void run(const SweepArgs &a, Shared &S, unsigned char *dyn, const IO<T> &io,
+                                             double &acc0, double &acc1) {
+    sweep<T, PM, SK, RY, NT>(a, S, dyn, io, acc0, acc1);
+  }
+};
+
 // The node's unit vector e_c, and the scaled Lanczos start vector, into a
 // window vector (pad columns zero).
-template <typename T>
+template <class Tile, typename T>
 static __device__ void unit_vector(const SweepArgs &a, Shared &S, T *v) {
-  const int NP = pair_cols(a.n), nw = (int)vec_points(a.n), nl = a.nloc;
-  const int c = (nl * a.n + nl) * NP + nl + (S.gi & 1);
+  const int NP = Tile::cols(a.n), nw = a.n * a.n * NP, nl = a.nloc;
+  const int c = (nl * a.n + nl) * NP + nl + Tile::shift(S);
   __syncthreads();
   for (int i = threadIdx.x; i < nw; i += blockDim.x) v[i] = (T)(i == c ? 1.0 : 0.0);
   __syncthreads();
 }
-template <typename T>
+template <class Tile, typename T>
 static __device__ void start_vector(const SweepArgs &a, Shared &S, T *v, double scale) {
-  const int n = a.n, NP = pair_cols(n), nw = (int)vec_points(n), sh = S.gi & 1;
+  const int n = a.n, NP = Tile::cols(n), nw = n * n * NP, sh = Tile::shift(S);
   __syncthreads();
   for (int i = threadIdx.x; i < nw; i += blockDim.x) {
     const int row = i / NP, x = i - row * NP - sh;  // row = z n + y, of the parity of z + y
@@ -1016,9 +1030,10 @@ static __device__ void start_vector(const SweepArgs &a, Shared &S, T *v, double 
 // extremes moved by no more than the tolerance, at most 500 steps) applies.
 // The projections chi^T W_m+1 the next gather needs follow from the recurrence
 // on the dot products of the sweep's output.
-template <typename T, int PM, bool LQ, int RY, int NT>
+template <class Tile, typename T, bool LQ>
 __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, double *pcur, double &lmin_out,
                         double &lmax_out, int &rows_out) {
+  constexpr int PM = Tile::PM;
   const int tid = threadIdx.x;
   const double nw = (double)a.n * a.n * a.n;
   T *Y = slot<T>(a, 0);
@@ -1028,15 +1043,15 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
   const int kmin = a.npl / 2 + 1;
   double d0 = 0.0, d1 = 0.0;
   if constexpr (LQ) {
-    unit_vector(a, S, Y);
+    unit_vector<Tile>(a, S, Y);
     centre_projections(a, S, pcur);  // W_0 = e_c
   } else {
-    start_vector(a, S, Y, s0);
+    start_vector<Tile>(a, S, Y, s0);
     // chi^T W_0 for W_0 = (1 + chk (-1)^(x+y+z)) / norm (sq.cpp:538-546, 993-1004
     // with chk = 0)
     IO<T> io;
     io.chk = chk;
-    sweep<T, PM, SK_ONES, RY, NT>(a, S, dyn, io, d0, d1);
+    Tile::template run<T, SK_ONES>(a, S, dyn, io, d0, d1);
     __syncthreads();
     for (int p = tid; p < S.n_pi; p += blockDim.x) {
       S.pw_cur[p] = s0 * S.p_nxt[p];
@@ -1070,7 +1085,7 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
     }
     d0 = 0.0;
     d1 = 0.0;
-    sweep<T, PM, SK_LZF, RY, NT>(a, S, dyn, io, d0, d1);
+    Tile::template run<T, SK_LZF>(a, S, dyn, io, d0, d1);
     sweep_sum2(S, d0, d1, a.nsweep);
     // b_m-1 = |W_m| and a_m = <W_m, H W_m> / b_m-1^2 (W_0 is normalised)
     const double bm = m == 0 ? 1.0 : sqrt(S.scal[0]);
@@ -1140,13 +1155,13 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
 }
 
 // Chebyshev moments mu_j = e_c^T T_j((H - chi)/zee) e_c / h^3 (sq.cpp:564-655).
-template <int PM, int RY, int NT>
+template <class Tile>
 __device__ void moments(const SweepArgs &a, Shared &S, unsigned char *dyn, double *pcur, double chi, double zee,
                         double *mu) {
   double *B0 = slot<double>(a, 0), *B1 = slot<double>(a, 1);
   double d0 = 0.0, d1 = 0.0;
   centre_projections(a, S, pcur);
-  unit_vector(a, S, B0);
+  unit_vector<Tile>(a, S, B0);
   {  // t_1 = (H e_c - chi e_c) / zee
     IO<double> io;
     io.vin = B0;
@@ -1154,7 +1169,7 @@ __device__ void moments(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
     io.out = B1;
     io.ca = chi;
     io.cb = zee;
-    sweep<double, PM, SK_CH, RY, NT>(a, S, dyn, io, d0, d1);
+    Tile::template run<double, SK_CH>(a, S, dyn, io, d0, d1);
   }
   __syncthreads();
   rotate(S, pcur);
@@ -1176,7 +1191,7 @@ __device__ void moments(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
       io.dbl = nq > q1;
       d0 = 0.0;
       d1 = 0.0;
-      sweep<double, PM, SK_CH, RY, NT>(a, S, dyn, io, d0, d1);
+      Tile::template run<double, SK_CH>(a, S, dyn, io, d0, d1);
       if (nq > q1) sweep_sum2(S, d0, d1, a.nsweep);
     }
     __syncthreads();
@@ -1235,7 +1250,7 @@ __device__ void node_forces(const SweepArgs &a, Shared &S, unsigned char *dyn, d
   T *B0 = slot<T>(a, 0), *B1 = slot<T>(a, 1);
   double *D = slot<double>(a, 2);
   double d0 = 0.0, d1 = 0.0;
-  unit_vector(a, S, B0);
+  unit_vector<PairTile<PM, RY, NT>>(a, S, B0);
   centre_projections(a, S, pcur);
   {  // t_1 = (H e_c - chi e_c) / zee; D = e_c Ci_0 / h^3 + t_1 Ci_1 / h^3
     IO<T> io;
@@ -1391,6 +1406,7 @@ static __device__ void quadrature_moments(const SweepArgs &a, Shared &S, int k, 
 // which sets the register budget per thread.
 template <int PM, int FORM, int MAXT, int RY, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) sweep_kernel(SweepArgs a) {
+  using Tile = PairTile<PM, RY, MAXT>;
   extern __shared__ __align__(128) unsigned char smem[];
   Shared &S = *reinterpret_cast<Shared *>(smem);
   unsigned char *dyn = smem + shared_fixed();
@@ -1417,7 +1433,7 @@ __global__ void __launch_bounds__(MAXT, MINB) sweep_kernel(SweepArgs a) {
     int rows = 0;
     double *mu = a.rho_pj + (size_t)node * (a.npl + 1);
     if constexpr (FORM == 2) {
-      lanczos<double, PM, true, RY, MAXT>(a, S, dyn, pcur, lmin, lmax, rows);
+      lanczos<Tile, double, true>(a, S, dyn, pcur, lmin, lmax, rows);
       const double chi = 0.5 * (lmax + lmin), zee = 0.5 * (lmax - lmin);
       if ((long long)rows <= (long long)a.n * a.n * a.n) quadrature_moments(a, S, rows, chi, zee, mu);
       else if (threadIdx.x == 0) atomicOr(a.status, ST_CAPACITY);
@@ -1426,13 +1442,13 @@ __global__ void __launch_bounds__(MAXT, MINB) sweep_kernel(SweepArgs a) {
     } else {
       using TL = typename std::conditional<FORM == 1, float, double>::type;
       if (FORM == 1) zero_planes(a, dyn, RY);  // FP32 values next
-      lanczos<TL, PM, false, RY, MAXT>(a, S, dyn, pcur, lmin, lmax, rows);
+      lanczos<Tile, TL, false>(a, S, dyn, pcur, lmin, lmax, rows);
       const double chi = (lmax + lmin) / 2, zee = (lmax - lmin) / 2;  // sq.cpp:564-565
       count_proj_points(a, S, rows + 1, 0);
       // moments stay FP64 in both forms: FP32 storage of the Chebyshev vectors
       // grows a rounding error injected at step i like (k - i) by step k
       if (FORM == 1) zero_planes(a, dyn, RY);  // FP64 values next
-      moments<PM, RY, MAXT>(a, S, dyn, pcur, chi, zee, mu);
+      moments<Tile>(a, S, dyn, pcur, chi, zee, mu);
       count_proj_points(a, S, a.npl / 2, 1);
     }
     if (threadIdx.x == 0) {
@@ -1476,8 +1492,9 @@ const void *pick_tile(int n, int ry) {
          : m == 896 ? K::template get<896, 1, 1>()
                     : K::template get<1024, 1, 1>();
 }
-// Shared-memory limit of a kernel for this launch and, on request, its
-// resident CTAs per SM.
+// Shared-memory limit of a kernel for a launch and, on request, its resident
+// CTAs per SM; tile_setup: of a default-tile kernel for the launch `a`.
+cudaError_t kernel_setup(const void *kernel, int threads, size_t smem, int *per_sm);
 cudaError_t tile_setup(const void *kernel, const SweepArgs &a, int *per_sm);
 
 }  // namespace sweep

@@ -6,10 +6,10 @@ The window edges are the smallest and largest of every tile (pairs of columns: w
 that start at odd and even columns of the halo'd block, the last pair half outside), for
 fields with one and with three projectors per slot.  Both kernels sum in FP64 in another
 order: a moment of order k carries about k^2 roundings of size 1e-16 (npl 16: 1e-13 with
-room), the bounds 1e-12 of the spectral range.  With three projectors per slot both
-kernels carry the projections of a Lanczos step by recurrence, whose rounding grows with
-the step count, so their bounds agree only within the stop: 1e-6 Ha of about 35 Ha, 3e-8,
-and the moments ten times that.  FP32 Lanczos vectors round at 6e-8, and
+room), the bounds 1e-12 of the spectral range.  LiH's Lanczos runs take up to 290 steps and
+stop on a plateau of the smallest eigenvalue, where a node's bound follows the order of
+every sum, so the bounds of two kernels agree only within the stop: 1e-6 Ha of about 35
+Ha, 3e-8, and the moments ten times that.  FP32 Lanczos vectors round at 6e-8, and
 the stop at 1e-3 Ha is met within that of each other.
 """
 from __future__ import annotations
@@ -70,7 +70,8 @@ def test_adjoint_matches_plane_kernel(system, nloc, npl):
 
 
 def test_layers_of_displaced_lih_fit():
-    """Displaced 64-atom LiH, where first fit in replica order needs five or six layers."""
+    """Displaced 64-atom LiH, where first fit in replica order needs five or six layers: the
+    fast forms and the forces run on the sweep kernel, the FP64 step where it is asked for."""
     from perf import cases
     from sqdft_b200 import sq
 
@@ -78,11 +79,81 @@ def test_layers_of_displaced_lih_fit():
     for seed in (0, 1, 2):
         s = cases.prepare(p, seed)
         with s["ctx"] as ctx:
+            ctx.set_node_kernel(sq.SQB_KERNEL_SWEEP)
             a = cases.run(s)
             assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_SWEEP
             ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
             b = cases.run(s)
         assert _rel(a["rho_pj"], b["rho_pj"]) <= 3e-7
+    for kind, form in (("sq", 1), ("sq", 2), ("forces", 0)):
+        s = cases.prepare(dict(p, kind=kind, form=form), 0)
+        with s["ctx"] as ctx:
+            cases.run(s)
+            assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_SWEEP
+
+
+def test_fp64_step_of_lih_keeps_its_kernel():
+    """64-atom LiH, 33^3 windows, a seed at which one node's stop moves by a step when the sums
+    change their order (Ci by 2e-7): the default step is the plane-streaming kernel's, bit for
+    bit, and so is the step of the graph mode and after an autotuner that does not apply."""
+    from perf import cases
+    from sqdft_b200 import sq
+
+    p = next(c for c in cases.listed() if c["name"] == "sq_fp64_w33_lih")
+    s = cases.prepare(p, 2)
+    with s["ctx"] as ctx:
+        a = cases.run(s)
+        assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_PLANE
+        with pytest.raises(sq.SQBError):
+            ctx.autotune_sweep(8)
+        ctx.set_graph(2)
+        g = cases.run(s)
+        ctx.set_graph(0)
+        ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
+        b = cases.run(s)
+    for k in b:
+        assert np.array_equal(a[k], b[k]) and np.array_equal(g[k], b[k]), k
+
+
+@pytest.mark.parametrize("per_cell,nloc,seed", [(14, 12, 2), (16, 14, 2), (12, 10, 2), (12, 10, 6)])
+def test_fp64_bounds_of_lih_keep_the_order_of_their_sums(per_cell, nloc, seed):
+    """8-atom LiH under first-fit layers, at seeds where bounds move by 2e-9 to 5e-9 of the
+    spectral range with the order of the sums: the bounds of the one-column tile (golden file
+    of the kernel it was first written as) to a few roundings of the range."""
+    from pathlib import Path
+
+    from perf import cases
+    from sqdft_b200 import sq
+
+    ref = np.load(Path(__file__).parent / "golden" / "lih_bounds_first_fit.npz")
+    s = cases.prepare(_params("sq", "lih", nloc, cells=1, per_cell=per_cell, block="5x4x3", kt=9.0), seed)
+    with s["ctx"] as ctx:
+        out = cases.run(s)
+        assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_SWEEP
+    for k in ("chi", "zee"):
+        assert _rel(out[k], ref[f"{per_cell}_{nloc}_{seed}_{k}"]) <= 1e-13, k
+
+
+@pytest.mark.parametrize("rows", [0, 3])
+@pytest.mark.parametrize("nloc", [4, 10, 15, 16, 19])
+def test_one_column_tile_matches_plane_kernel(nloc, rows):
+    """8-atom LiH, where first fit needs four layers: windows with a warp per row group (up to
+    31 wide) and with packed columns (from 33 on), and n mod 3 of 0, 1 and 2."""
+    from perf import cases
+    from sqdft_b200 import sq
+
+    if rows == 3 and nloc > 16:
+        pytest.skip("three rows cover windows up to 33 wide")
+    s = cases.prepare(_params("sq", "lih", nloc, cells=1, per_cell=20), 3)
+    with s["ctx"] as ctx:
+        ctx.set_sweep_rows(rows)
+        a = cases.run(s)
+        assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_SWEEP
+        ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
+        b = cases.run(s)
+    for k in ("chi", "zee"):
+        assert _rel(a[k], b[k]) <= 3e-8, k
+    assert _rel(a["rho_pj"], b["rho_pj"]) <= 3e-7
 
 
 @pytest.mark.parametrize("grid_kind", ["uniform", "coarse", "octaves"])
