@@ -322,8 +322,16 @@ int sqb_moments_at(sqb_ctx *ctx, const double *chi, const double *zee, double *r
  * sqb_set_veff) and, when g_atoms is not NULL, g_atoms = dL/dR [n_atm][3]
  * (type-major, the layout of sqb_forces_nonlocal) through the projector
  * tables, with the spectral bounds chi, zee of the last moments held fixed.
- * Computed by the reverse Chebyshev (Clenshaw) recursion with checkpoints
- * every 8 recursion vectors; the projector derivatives dchi/dR are central
+ * On the sweep kernel (sqb_set_node_kernel) the npl recursion vectors of a
+ * node are kept and the gradient is a quadratic form of them: npl (n + 1) n^2
+ * doubles for each resident CTA (n the window edge; 1.5 GB at 27^3 and npl
+ * 64, 12.3 GB at 43^3 and npl 128), held until sqb_destroy, but never more
+ * than a quarter of the device's free memory: fewer CTAs share the nodes
+ * then, and where a quarter of the SMs would not get their vectors the call
+ * runs on the plane-streaming kernel, as it does where the sweep kernel does
+ * not cover the system (sqb_stats.node_kernel tells).  There the reverse
+ * Chebyshev (Clenshaw) recursion runs with checkpoints every 8 recursion
+ * vectors.  The projector derivatives dchi/dR are central
  * differences (step 1e-4 bohr) of the projector tables.  Contributions of
  * different nodes to one Veff point or atom are added with atomics, so the
  * outputs vary between runs at rounding level.  No counterpart in the

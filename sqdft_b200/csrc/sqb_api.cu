@@ -1867,71 +1867,112 @@ static int ensure_dtab(sqb_ctx *c) {
 
 }  // extern "C"
 
-// Moment adjoint on the plane-streaming kernel (node_vjp): buffers, then the
-// weights dL/dmu [N][npl+1] filled by `fill` into the device array it is
-// given (a copy from the host, or a kernel), then the launch.
+// The adjoint's buffer of window vectors, at least `need` bytes; false (and no
+// buffer) where the device does not have them.
+static bool reserve_vjp(sqb_ctx *c, size_t need) {
+  if (c->vjp_bytes >= need) return true;
+  if (c->d_vjp) cudaFree(c->d_vjp);
+  c->d_vjp = nullptr;
+  c->vjp_bytes = 0;
+  if (cudaMalloc((void **)&c->d_vjp, need) != cudaSuccess) {
+    cudaGetLastError();
+    c->d_vjp = nullptr;
+    return false;
+  }
+  c->vjp_bytes = need;
+  return true;
+}
+
+// The vectors of the sweep kernel's adjoint: npl window vectors for each of its
+// *grid CTAs (27^3 windows, npl 64: 10 MB a CTA, 1.5 GB in all; 43^3, npl 128:
+// 83 MB, 12.3 GB), which stay with the context.  At most a quarter of the
+// device's free memory goes into them: past that fewer CTAs share the nodes.
+// Below a quarter of the SMs the plane-streaming kernel takes over (*grid 0),
+// whose checkpoints need a third of the memory and whose reverse recursion
+// three times the matvecs.
+static int reserve_sweep_vjp(sqb_ctx *c, size_t per, size_t fixed, int *grid) {
+  const int few = std::min(c->sms, c->nnode);
+  auto bytes = [&](int g) { return (per * g + fixed) * sizeof(double); };
+  int g = *grid;
+  if (c->vjp_bytes < bytes(g)) {
+    size_t avail = 0, total = 0;
+    CK(cudaMemGetInfo(&avail, &total));
+    const size_t cap = std::max((avail + c->vjp_bytes) / 4, c->vjp_bytes);
+    while (g > 0 && bytes(g) > cap) g--;
+    while (4 * g >= few && !reserve_vjp(c, bytes(g))) g /= 2;
+    if (4 * g < few) g = 0;
+  }
+  *grid = g;
+  return SQB_OK;
+}
+
+// Moment adjoint on the sweep kernel where it covers the context and its
+// vectors can be had, else on the plane-streaming kernel (node_vjp): buffers,
+// the vectors last, then the weights dL/dmu [N][npl+1] filled by `fill` into
+// the device array it is given (a copy from the host, or a kernel), then the
+// launch.
 template <typename Fill>
 static int moments_vjp(sqb_ctx *c, Fill fill, double *g_veff, double *g_atoms) {
   const size_t N = c->nnode, K = c->g.npl + 1;
   const size_t nw = (size_t)c->n * c->n * c->n;
-  const size_t ext = (size_t)c->ex * c->ey * c->ez;
-  const int nseg = (c->g.npl + VJP_K - 1) / VJP_K;
-  size_t per = ((size_t)(2 * nseg + VJP_K + 4) * nw + (size_t)nseg * MAXP + 31) & ~size_t(31);  // doubles
-  int grid = c->sms * (c->ctas_per_sm > 0 ? c->ctas_per_sm : 1);
-  if ((size_t)grid > N) grid = (int)N;
-  auto reserve = [&](size_t need) {
-    if (c->vjp_bytes >= need) return true;
-    if (c->d_vjp) cudaFree(c->d_vjp);
-    c->d_vjp = nullptr;
-    c->vjp_bytes = 0;
-    if (cudaMalloc((void **)&c->d_vjp, need) != cudaSuccess) {
-      cudaGetLastError();
-      c->d_vjp = nullptr;
-      return false;
-    }
-    c->vjp_bytes = need;
-    return true;
-  };
-  // The sweep kernel where it covers the system and its npl window vectors per
-  // CTA can be had (27^3 windows, npl 64: 1.5 GB in all; the plane-streaming
-  // kernel's checkpoints take 0.6 GB and its reverse recursion three times the
-  // matvecs), else the plane-streaming kernel.
+  const size_t ext = (size_t)c->ex * c->ey * c->ez, fixed = N * K + ext;
   int rc = c->node_kernel == SQB_KERNEL_PLANE ? SQB_OK : ensure_layers(c);
   if (rc) return rc;
   bool sw = c->node_kernel != SQB_KERNEL_PLANE && c->lay_state == 1;
+  if (g_atoms) {
+    rc = ensure_dtab(c);
+    if (rc) return rc;
+  }
+  const size_t n3 = (size_t)3 * std::max(c->n_atm, 1);
+  auto reserve_atoms = [&](size_t doubles) {
+    if (c->vjp_at_bytes >= doubles * sizeof(double)) return SQB_OK;
+    if (c->d_vjp_at) cudaFree(c->d_vjp_at);
+    c->d_vjp_at = nullptr;
+    c->vjp_at_bytes = 0;
+    CK(cudaMalloc((void **)&c->d_vjp_at, doubles * sizeof(double)));
+    c->vjp_at_bytes = doubles * sizeof(double);
+    return SQB_OK;
+  };
   SweepArgs sa;
+  size_t per = 0, per_at = 0;  // doubles per CTA
+  int grid = 0;
   if (sw) {
     fill_sweep_args(c, c->d_nodes, c->nnode, sa);
     int per_sm = 0;
     CK(sweep_vjp_per_sm(sa, &per_sm));
-    const int g = std::max(1, std::min(c->sms * per_sm, c->nnode));
-    const size_t p = sweep_vjp_doubles(c->n, c->g.npl);
-    sw = reserve((p * g + N * K + ext) * sizeof(double));
-    if (sw) {
-      grid = g;
-      per = p;
-      rc = ensure_sweep_scratch(c, grid, &sa.scratch_stride);
-      if (rc) return rc;
-      sa.scratch = c->d_scratch;
+    if (sweep_grid(c, per_sm, sa, &grid) != SQB_OK) {  // no room for the scratch
+      cudaGetLastError();
+      sw = false;
     }
   }
-  if (!sw && !reserve((per * grid + N * K + ext) * sizeof(double))) return SQB_ERR_CUDA;
+  if (sw) {
+    if (g_atoms) {
+      rc = reserve_atoms(n3);
+      if (rc) return rc;
+    }
+    per = sweep_vjp_doubles(c->n, c->g.npl);
+    rc = reserve_sweep_vjp(c, per, fixed, &grid);
+    if (rc) return rc;
+    sw = grid > 0;
+  }
+  if (!sw) {
+    const int nseg = (c->g.npl + VJP_K - 1) / VJP_K;
+    per = ((size_t)(2 * nseg + VJP_K + 4) * nw + (size_t)nseg * MAXP + 31) & ~size_t(31);
+    grid = c->sms * (c->ctas_per_sm > 0 ? c->ctas_per_sm : 1);
+    if ((size_t)grid > N) grid = (int)N;
+    per_at = (size_t)(4 * VJP_K + 12) * MAXP;
+    if (g_atoms) {
+      rc = reserve_atoms(per_at * grid + n3);
+      if (rc) return rc;
+    }
+    if (!reserve_vjp(c, (per * grid + fixed) * sizeof(double))) return SQB_ERR_CUDA;
+  }
+  c->stats.node_kernel = sw ? SQB_KERNEL_SWEEP : SQB_KERNEL_PLANE;
   double *d_scr = c->d_vjp, *d_g = d_scr + per * grid, *d_out = d_g + N * K;
-  const size_t per_at = (size_t)(4 * VJP_K + 12) * MAXP;  // doubles per CTA
   double *d_gat = nullptr;
   if (g_atoms) {
-    int rc0 = ensure_dtab(c);
-    if (rc0) return rc0;
-    const size_t need_at = (per_at * grid + (size_t)3 * std::max(c->n_atm, 1)) * sizeof(double);
-    if (c->vjp_at_bytes < need_at) {
-      if (c->d_vjp_at) cudaFree(c->d_vjp_at);
-      c->d_vjp_at = nullptr;
-      c->vjp_at_bytes = 0;
-      CK(cudaMalloc((void **)&c->d_vjp_at, need_at));
-      c->vjp_at_bytes = need_at;
-    }
     d_gat = c->d_vjp_at + per_at * grid;
-    CK(cudaMemsetAsync(d_gat, 0, (size_t)3 * std::max(c->n_atm, 1) * sizeof(double), c->stream));
+    CK(cudaMemsetAsync(d_gat, 0, n3 * sizeof(double), c->stream));
   }
   rc = fill(d_g);
   if (rc) return rc;

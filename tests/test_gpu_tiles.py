@@ -40,8 +40,11 @@ def _both(p, seed=3):
     with s["ctx"] as ctx:
         ctx.set_node_kernel(sq.SQB_KERNEL_SWEEP)
         a = cases.run(s)
+        assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_SWEEP
         ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
-        return a, cases.run(s)
+        b = cases.run(s)
+        assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_PLANE
+        return a, b
 
 
 @pytest.mark.parametrize("system", ["al", "lih"])
@@ -65,6 +68,39 @@ def test_tiles_match_plane_kernel(system, nloc):
 def test_adjoint_matches_plane_kernel(system, nloc, npl):
     """Block remainders of the quadratic form (16 vectors, 8 at a time), one block and several."""
     (gv, ga), (gv0, ga0) = _both(_params("vjp", system, nloc, npl=npl, per_cell=20))
+    assert _rel(gv, gv0) <= 1e-12
+    assert _rel(ga, ga0) <= 1e-11
+
+
+@pytest.mark.parametrize("left,kernel", [(8.0e9, 2), (3.6e9, 1)])
+def test_adjoint_where_memory_is_short(left, kernel):
+    """35^3 windows, npl 64, 150 nodes: 3.4 GB of vectors for 148 CTAs.  With 8 GB free fewer CTAs
+    take a quarter of it; with 3.6 GB, where the vectors alone would fit but not the scratch
+    beside them, the call runs on the plane-streaming kernel."""
+    import torch
+
+    from perf import cases
+    from sqdft_b200 import sq
+
+    p = _params("vjp", "al", 17, npl=64, per_cell=20, block="6x5x5")
+    s = cases.prepare(p, 3)
+    with s["ctx"] as ctx:
+        ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
+        gv0, ga0 = cases.run(s)
+    s = cases.prepare(p, 3)
+    with s["ctx"] as ctx:
+        torch.cuda.empty_cache()
+        held = torch.empty(int(torch.cuda.mem_get_info()[0] - left), dtype=torch.uint8, device="cuda")
+        try:
+            free = torch.cuda.mem_get_info()[0]
+            gv, ga = cases.run(s)
+            taken = free - torch.cuda.mem_get_info()[0]
+        finally:
+            del held
+            torch.cuda.empty_cache()
+        assert ctx.stats()["node_kernel"] == kernel
+    # the vectors' quarter, or the plane-streaming kernel's checkpoints (1.44 GB); 0.65 GB of scratch and tables
+    assert taken <= (left / 4 if kernel == sq.SQB_KERNEL_SWEEP else 1.45e9) + 0.75e9
     assert _rel(gv, gv0) <= 1e-12
     assert _rel(ga, ga0) <= 1e-11
 
