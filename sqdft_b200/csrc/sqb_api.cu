@@ -128,10 +128,13 @@ struct sqb_ctx {
 
 namespace {
 
+// (The error is cleared: one that leaves the device usable, as a failed
+// allocation, must not come back from the next launch's check.)
 #define CK(x)                                    \
   do {                                           \
     cudaError_t e_ = (x);                        \
     if (e_ != cudaSuccess) {                     \
+      cudaGetLastError();                        \
       std::fprintf(stderr, "sqdft_b200: %s at %s:%d\n", cudaGetErrorString(e_), __FILE__, __LINE__); \
       return SQB_ERR_CUDA;                       \
     }                                            \
@@ -200,6 +203,7 @@ int ensure_tmp(sqb_ctx *c, size_t bytes) {
   if (c->tmp_bytes >= bytes) return SQB_OK;
   if (c->d_tmp) cudaFree(c->d_tmp);
   c->d_tmp = nullptr;
+  c->tmp_bytes = 0;  // (a failed allocation leaves no size behind)
   CK(cudaMalloc((void **)&c->d_tmp, bytes));
   c->tmp_bytes = bytes;
   return SQB_OK;
@@ -218,6 +222,7 @@ int ensure_scratch(sqb_ctx *c, int grid) {
     drop_graph(c);  // captured launches hold the old buffer's address
     if (c->d_scratch) cudaFree(c->d_scratch);
     c->d_scratch = nullptr;
+    c->scratch_bytes = 0;  // (a failed allocation leaves no size behind)
     CK(cudaMalloc((void **)&c->d_scratch, need));
     c->scratch_bytes = need;
   }
@@ -1940,10 +1945,7 @@ static int moments_vjp(sqb_ctx *c, Fill fill, double *g_veff, double *g_atoms) {
     fill_sweep_args(c, c->d_nodes, c->nnode, sa);
     int per_sm = 0;
     CK(sweep_vjp_per_sm(sa, &per_sm));
-    if (sweep_grid(c, per_sm, sa, &grid) != SQB_OK) {  // no room for the scratch
-      cudaGetLastError();
-      sw = false;
-    }
+    sw = sweep_grid(c, per_sm, sa, &grid) == SQB_OK;  // (not where there is no room for the scratch)
   }
   if (sw) {
     if (g_atoms) {
@@ -2303,6 +2305,7 @@ int ensure_local_fields(sqb_ctx *c, double **f, double **phi, double **partial) 
   if (c->loc_fields_bytes < need) {
     if (c->d_loc_fields) cudaFree(c->d_loc_fields);
     c->d_loc_fields = nullptr;
+    c->loc_fields_bytes = 0;  // (a failed allocation leaves no size behind)
     CK(cudaMalloc((void **)&c->d_loc_fields, need));
     c->loc_fields_bytes = need;
   }
@@ -2500,6 +2503,7 @@ int sqb_forces_local(sqb_ctx *c, const double *phi, const double *vc, const doub
     if (c->loc_scr_bytes < need) {
       if (c->d_loc_scr) cudaFree(c->d_loc_scr);
       c->d_loc_scr = nullptr;
+      c->loc_scr_bytes = 0;  // (a failed allocation leaves no size behind)
       CK(cudaMalloc((void **)&c->d_loc_scr, need));
       c->loc_scr_bytes = need;
     }

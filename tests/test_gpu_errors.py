@@ -126,3 +126,34 @@ def test_bounded_stage_wait_runs_out_cleanly(golden):
         m = ctx.lanczos_moments()
     assert np.abs(m["chi"] - ref["chi"]).max() <= 1e-10
     assert np.abs(m["zee"] - ref["zee"]).max() <= 1e-10
+
+
+def test_a_failed_scratch_allocation_leaves_the_context_usable():
+    """Scratch for eight CTAs, then for 148 (39^3 windows, 0.28 GB) with 0.1 GB of device memory
+    left: the call returns SQB_ERR_CUDA, a smaller one allocates its own buffer again, and with
+    the memory back the step runs."""
+    import torch
+
+    from perf import cases
+    from sqdft_b200 import sq
+
+    p = dict(kind="sq", system="al", form=0, cells=2, per_cell=20, block="6x5x5", nloc=19, npl=4, kt=5.0)
+    s = cases.prepare(p, 3)
+    with s["ctx"] as ctx:
+        ctx.set_veff(s["veff"])
+        ctx.set_node_kernel(sq.SQB_KERNEL_PLANE)
+        ctx.autotune(8)
+        torch.cuda.empty_cache()
+        held = torch.empty(int(torch.cuda.mem_get_info()[0] - 1.0e8), dtype=torch.uint8, device="cuda")
+        try:
+            with pytest.raises(sq.SQBError) as err:
+                ctx.lanczos_moments()
+            assert err.value.code == 2  # SQB_ERR_CUDA
+            ctx.autotune(8)
+        finally:
+            del held
+            torch.cuda.empty_cache()
+        a = ctx.lanczos_moments()
+        ctx.set_node_kernel(sq.SQB_KERNEL_SWEEP)
+        b = ctx.lanczos_moments()
+    assert np.abs(a["chi"] - b["chi"]).max() <= 1e-10
