@@ -188,13 +188,14 @@ int reduce(sqb_ctx *c, double *v, int count, int op) {
 }
 
 int status_to_err(int st) {
+  // a wait that ran out leaves values that were never written, so whatever else is set follows from it
+  if (st & ST_WAIT_LIMIT) return SQB_ERR_CUDA;
   if (st & ST_CAPACITY) return SQB_ERR_CAPACITY;
   if (st & ST_FSLOTS) return SQB_ERR_CAPACITY;
   if (st & ST_SPLINE_RANGE) return SQB_ERR_SPLINE_RANGE;
   if (st & ST_NONFINITE) return SQB_ERR_NONFINITE;
   // ST_LANCZOS_MAXITER is a warning: the reference prints and carries on with
   // the last Ritz values (sq.cpp:1073-1074); the nodes are counted in the stats.
-  if (st & ST_WAIT_LIMIT) return SQB_ERR_CUDA;
   if (st & ST_BOUNDS) return SQB_ERR_BOUNDS;
   return SQB_OK;
 }
