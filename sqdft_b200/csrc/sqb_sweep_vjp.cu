@@ -90,20 +90,28 @@ __device__ void node_vjp(const SweepArgs &a, Shared &S, unsigned char *dyn, doub
   // atoms' sums on the way, so the vectors (1.5 GB at 27^3 windows and npl 64)
   // are not read again for each ball.
   const unsigned dummy = (unsigned)a.n_gproj;
+  // (a ball with fewer than PM projectors reads on into the next one's Cl, or
+  // past the last into the weights; nothing reads those sums)
+  const int nC = MAXP * npl + vjp_weights(npl);
+  const long long nV = a.evol / a.ex * a.gex;  // values of g_veff
+  (void)nC;
+  (void)nV;
   for (int i = tid; i < NW / 2; i += blockDim.x) {
     const int row = i / HX, x = 2 * (i - row * HX) - sh, z = row / n, y = row - z * n;
     const double *tp = T + 2 * i;
+    const long long nT = (long long)npl * NW;
+    (void)nT;
     const bool in0 = x >= 0, in1 = x + 1 < n;
     int off[KL][2];
     double2 u[KL][PM];
     if (at) {
       const ulonglong2 id = __ldg(reinterpret_cast<const ulonglong2 *>(
-          a.lay_id + ((S.gk + z) * a.ey + S.gj + y) * a.ex + S.gi + x));
+          a.lay_id + SQB_IDX(((S.gk + z) * a.ey + S.gj + y) * a.ex + S.gi + x, a.evol - 1, a.status)));
 #pragma unroll
       for (int k = 0; k < KL; k++) {
         const unsigned i0 = lay_of(id.x, k), i1 = lay_of(id.y, k);
-        off[k][0] = in0 && i0 != dummy ? *reinterpret_cast<const int *>(pcur + i0) * npl : -1;
-        off[k][1] = in1 && i1 != dummy ? *reinterpret_cast<const int *>(pcur + i1) * npl : -1;
+        off[k][0] = in0 && i0 != dummy ? *reinterpret_cast<const int *>(pcur + SQB_IDX(i0, a.n_gproj, a.status)) * npl : -1;
+        off[k][1] = in1 && i1 != dummy ? *reinterpret_cast<const int *>(pcur + SQB_IDX(i1, a.n_gproj, a.status)) * npl : -1;
 #pragma unroll
         for (int q = 0; q < PM; q++) u[k][q] = make_double2(0.0, 0.0);
       }
@@ -113,8 +121,8 @@ __device__ void node_vjp(const SweepArgs &a, Shared &S, unsigned char *dyn, doub
       for (int k = 0; k < KL; k++) {
 #pragma unroll
         for (int q = 0; q < PM; q++) {
-          if (off[k][0] >= 0) u[k][q].x += Cl[off[k][0] + q * npl + l] * t.x;
-          if (off[k][1] >= 0) u[k][q].y += Cl[off[k][1] + q * npl + l] * t.y;
+          if (off[k][0] >= 0) u[k][q].x += Cl[SQB_IDX(off[k][0] + q * npl + l, nC, a.status)] * t.x;
+          if (off[k][1] >= 0) u[k][q].y += Cl[SQB_IDX(off[k][1] + q * npl + l, nC, a.status)] * t.y;
         }
       }
     };
@@ -123,7 +131,7 @@ __device__ void node_vjp(const SweepArgs &a, Shared &S, unsigned char *dyn, doub
       double2 tk[VB];
 #pragma unroll
       for (int k = 0; k < VB; k++)
-        tk[k] = K0 + k < npl ? __ldcg(reinterpret_cast<const double2 *>(tp + (size_t)(K0 + k) * NW)) : make_double2(0.0, 0.0);
+        tk[k] = K0 + k < npl ? __ldcg(reinterpret_cast<const double2 *>(tp + SQB_IDX((size_t)(K0 + k) * NW, nT - 2 * i - 1, a.status))) : make_double2(0.0, 0.0);
 #pragma unroll
       for (int k = 0; k < VB; k++) {
         const double w = K0 + k ? 2.0 : 1.0;
@@ -145,7 +153,7 @@ __device__ void node_vjp(const SweepArgs &a, Shared &S, unsigned char *dyn, doub
           cx += s * tk[k].x;
           cy += s * tk[k].y;
         }
-        const double s = Sw[2 * K0 + 2 * l + 1];
+        const double s = Sw[SQB_IDX(2 * K0 + 2 * l + 1, nS, a.status)];
         gx += tk[l].x * (2.0 * cx + s * tk[l].x);
         gy += tk[l].y * (2.0 * cy + s * tk[l].y);
       }
@@ -154,12 +162,12 @@ __device__ void node_vjp(const SweepArgs &a, Shared &S, unsigned char *dyn, doub
         double2 tl[VL];
 #pragma unroll
         for (int l = 0; l < VL; l++)
-          tl[l] = L0 + l < npl ? __ldcg(reinterpret_cast<const double2 *>(tp + (size_t)(L0 + l) * NW)) : make_double2(0.0, 0.0);
+          tl[l] = L0 + l < npl ? __ldcg(reinterpret_cast<const double2 *>(tp + SQB_IDX((size_t)(L0 + l) * NW, nT - 2 * i - 1, a.status))) : make_double2(0.0, 0.0);
 #pragma unroll
         for (int l = 0; l < VL; l++) {
           tl[l].x *= 2.0;
           tl[l].y *= 2.0;
-          const double *s = Sw + K0 + L0 + l + 1;
+          const double *s = Sw + SQB_IDX(K0 + L0 + l + 1, nS - VB + 1, a.status);
           double cx = 0.0, cy = 0.0;
 #pragma unroll
           for (int k = 0; k < VB; k++) {
@@ -174,15 +182,16 @@ __device__ void node_vjp(const SweepArgs &a, Shared &S, unsigned char *dyn, doub
       }
     }
     // the window of node (gi, gj, gk) starts there in the halo'd block
-    double *ve = a.g_veff + ((size_t)(S.gk + z) * a.ey + (S.gj + y)) * a.gex + (S.gi + x);
-    if (in0) atomicAdd(ve, gx * iz);
-    if (in1) atomicAdd(ve + 1, gy * iz);
+    const long long v0 = ((long long)(S.gk + z) * a.ey + (S.gj + y)) * a.gex + (S.gi + x);
+    if (in0) atomicAdd(a.g_veff + SQB_IDX(v0, nV, a.status), gx * iz);
+    if (in1) atomicAdd(a.g_veff + SQB_IDX(v0 + 1, nV, a.status), gy * iz);
     if (at) {
 #pragma unroll
       for (int k = 0; k < KL; k++)
 #pragma unroll
         for (int q = 0; q < PM; q++)
-          *reinterpret_cast<double2 *>(uf + (size_t)(k * PM + q) * NW + 2 * i) = u[k][q];
+          *reinterpret_cast<double2 *>(uf + SQB_IDX((size_t)(k * PM + q) * NW + 2 * i, (size_t)KL * PM * NW - 1, a.status)) =
+              u[k][q];
     }
   }
   if (!at) return;
@@ -204,8 +213,9 @@ __device__ void node_vjp(const SweepArgs &a, Shared &S, unsigned char *dyn, doub
       const int yz = i / bx, x = x0 + i - yz * bx, zz = yz / by, y = y0 + yz - zz * by, z = z0 + zz;
       const int w = z * VP + y * NP + x + sh;
       for (int q = 0; q < np; q++) {
-        const double u = uk[(size_t)q * NW + w];
-        const double *d = U + (size_t)(q * Sd + oz + z) * sp2 + (oy + y) * Sd + ox + x;
+        const double u = uk[SQB_IDX((size_t)q * NW + w, (size_t)PM * NW, a.status)];
+        const long long o = (long long)(q * Sd + oz + z) * sp2 + (oy + y) * Sd + ox + x;
+        const double *d = U + SQB_IDX(o, a.dtab_stride - a.rep_off[r], a.status);
         ax += u * d[0];
         ay += u * d[a.dtab_stride];
         az += u * d[2 * a.dtab_stride];
