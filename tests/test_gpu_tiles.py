@@ -31,13 +31,14 @@ def _params(kind, system, nloc, form=0, npl=16, **kw):
     return d
 
 
-def _both(p, seed=3):
-    """Outputs of the sweep kernel and of the plane-streaming kernel on the same inputs."""
+def _both(p, seed=3, rows=0):
+    """Outputs of the sweep kernel (`rows` of sqb_set_sweep_rows) and of the plane-streaming kernel on the same inputs."""
     from perf import cases
     from sqdft_b200 import sq
 
     s = cases.prepare(p, seed)
     with s["ctx"] as ctx:
+        ctx.set_sweep_rows(rows)
         ctx.set_node_kernel(sq.SQB_KERNEL_SWEEP)
         a = cases.run(s)
         assert ctx.stats()["node_kernel"] == sq.SQB_KERNEL_SWEEP
@@ -47,20 +48,40 @@ def _both(p, seed=3):
         return a, b
 
 
-@pytest.mark.parametrize("system", ["al", "lih"])
-@pytest.mark.parametrize("nloc", [4, 9, 10, 13, 15, 16, 17, 19, 21])
-def test_tiles_match_plane_kernel(system, nloc):
-    if system == "lih" and nloc == 9:
-        pytest.skip("two species at this spacing need more than four layers")
+def _check_tiles(system, nloc, rows=0, **kw):
+    kw.setdefault("per_cell", 20 if system == "lih" or nloc > 13 else 12)
     for form in (0, 1, 2):
-        a, b = _both(_params("sq", system, nloc, form, per_cell=20 if system == "lih" or nloc > 13 else 12))
+        a, b = _both(_params("sq", system, nloc, form, **kw), rows=rows)
         tol = 1e-6 if form == 1 else 3e-8 if system == "lih" else 1e-12
         for k in ("chi", "zee"):
             assert _rel(a[k], b[k]) <= tol, (form, k)
         assert _rel(a["rho_pj"], b["rho_pj"]) <= 10 * tol, form
     for form in (0, 1):
-        a, b = _both(_params("forces", system, nloc, form, per_cell=20 if system == "lih" or nloc > 13 else 12))
+        a, b = _both(_params("forces", system, nloc, form, **kw), rows=rows)
         assert _rel(a, b) <= (1e-5 if form else 1e-11), form
+
+
+@pytest.mark.parametrize("system", ["al", "lih"])
+@pytest.mark.parametrize("nloc", [4, 9, 10, 13, 15, 16, 17, 19, 21])
+def test_tiles_match_plane_kernel(system, nloc):
+    _check_tiles(system, nloc)
+
+
+@pytest.mark.parametrize("system", ["al", "lih"])
+@pytest.mark.parametrize("nloc", [4, 8, 9, 16])
+def test_three_row_tiles_match_plane_kernel(system, nloc):
+    """Three rows per thread: edges 9, 17, 19 and 33, n mod 3 = 0, 2, 1 and the widest."""
+    _check_tiles(system, nloc, rows=3)
+
+
+@pytest.mark.parametrize("system", ["al", "lih"])
+def test_many_nodes_per_cta(system):
+    """512 nodes of 9^3 windows, more than resident CTAs: what a CTA carries from one node to the
+    next, of the other parity or not."""
+    _check_tiles(system, 4, block="8x8x8", per_cell=20)
+    (gv, ga), (gv0, ga0) = _both(_params("vjp", system, 4, npl=20, per_cell=20, block="8x8x8"))
+    assert _rel(gv, gv0) <= 1e-12
+    assert _rel(ga, ga0) <= 1e-11
 
 
 @pytest.mark.parametrize("system,nloc,npl", [("al", 4, 4), ("al", 9, 16), ("al", 10, 20), ("al", 15, 36),
@@ -68,6 +89,14 @@ def test_tiles_match_plane_kernel(system, nloc):
 def test_adjoint_matches_plane_kernel(system, nloc, npl):
     """Block remainders of the quadratic form (16 vectors, 8 at a time), one block and several."""
     (gv, ga), (gv0, ga0) = _both(_params("vjp", system, nloc, npl=npl, per_cell=20))
+    assert _rel(gv, gv0) <= 1e-12
+    assert _rel(ga, ga0) <= 1e-11
+
+
+@pytest.mark.parametrize("system,nloc,npl", [("al", 4, 20), ("al", 8, 16), ("al", 9, 16), ("al", 16, 12),
+                                             ("lih", 4, 20), ("lih", 8, 16), ("lih", 9, 16), ("lih", 16, 12)])
+def test_three_row_adjoint_matches_plane_kernel(system, nloc, npl):
+    (gv, ga), (gv0, ga0) = _both(_params("vjp", system, nloc, npl=npl, per_cell=20), rows=3)
     assert _rel(gv, gv0) <= 1e-12
     assert _rel(ga, ga0) <= 1e-11
 
