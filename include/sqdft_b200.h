@@ -128,8 +128,8 @@ typedef struct sqb_stats {
                                       the 500-iteration cap (sq.cpp:1073-1074 prints them) */
   long long proj_points_window; /* as proj_points, with each ball clipped to the window (the
                                    projector values a matvec reads) */
-  int node_kernel;           /* kernel of the last Lanczos + moments work: SQB_KERNEL_PLANE or
-                                SQB_KERNEL_SWEEP */
+  int node_kernel;           /* kernel of the last Lanczos + moments work, nonlocal forces or adjoint:
+                                SQB_KERNEL_PLANE or SQB_KERNEL_SWEEP */
   double ms_charge_density;  /* kernels of the last sqb_charge_density */
   double ms_forces_local;    /* kernels of the last sqb_forces_local */
 } sqb_stats;
@@ -177,15 +177,15 @@ int sqb_set_launch(sqb_ctx *ctx, int ctas_per_sm, int cols_per_thread);
  * balls split into four such layers (the FCC sublattices) with at most three
  * projectors per type.  SQB_KERNEL_PLANE: the plane-streaming kernel with
  * per-window box lists, any system.  SQB_KERNEL_AUTO (default): the sweep
- * kernel where it covers the system, but for the FP64 SQ step of systems with
- * more than one projector per ball that split only by saturation colouring
- * and not by first fit in replica order (64-atom LiH), which stays on the
- * plane-streaming kernel.  Results agree to rounding, which the Lanczos stop
- * can amplify: a run of 200 steps and more (LiH) that stops on a plateau of
- * the smallest eigenvalue ends at a bound that moves by up to the stop with
- * the order of the sums, so such a system keeps its kernel unless
- * SQB_KERNEL_SWEEP asks for the faster one.  The nonlocal forces and the
- * adjoint run on the sweep kernel where it covers the system; sqb_moments_at,
+ * kernel where it covers the system.  Results agree to rounding; a Lanczos run
+ * of more than about 6.5 window edges (LiH; Al stops after 1.6 to 2.7)
+ * amplifies it, and its bounds can move by up to the stop with the order of
+ * the sums.  In the FP64 step of systems with more than one projector per ball
+ * the sweep kernel therefore repeats the nodes whose runs pass six edges in a
+ * second launch that keeps one order: the plane-streaming kernel's, or under
+ * layers found by first fit in replica order that of a tile with one column
+ * per thread.  The nonlocal
+ * forces and the adjoint follow the same choice; sqb_moments_at,
  * sqb_hsub_times_vec and sqb_lanczos_moments_noalloc run the plane-streaming
  * kernel.  No counterpart in the reference. */
 #define SQB_KERNEL_AUTO 0
@@ -193,8 +193,7 @@ int sqb_set_launch(sqb_ctx *ctx, int ctas_per_sm, int cols_per_thread);
 #define SQB_KERNEL_SWEEP 2
 int sqb_set_node_kernel(sqb_ctx *ctx, int kernel);
 /* Tile of the sweep kernel's threads: 0 or 2 the default one (a pair of window
- * columns and one row per thread; one column and two rows in the FP64 SQ step
- * of systems with more than one projector per ball), 3 three rows (fewer
+ * columns and one row per thread), 3 a pair of columns and three rows (fewer
  * threads, more registers each; windows up to 33 wide).  Results agree to
  * rounding (the block reductions sum in another order). */
 int sqb_set_sweep_rows(sqb_ctx *ctx, int rows);

@@ -85,7 +85,8 @@ struct sqb_ctx {
 
   unsigned char *d_scratch = nullptr;
   size_t scratch_stride = 0, scratch_bytes = 0;
-  int *d_counter = nullptr, *d_nodes = nullptr, *d_status = nullptr, *d_iters = nullptr;
+  int redo_n = 0;  // nodes d_redo holds
+  int *d_counter = nullptr, *d_redo = nullptr, *d_nodes = nullptr, *d_status = nullptr, *d_iters = nullptr;
   unsigned long long *d_proj_points = nullptr;
   double *d_chi = nullptr, *d_zee = nullptr, *d_rho_pj = nullptr, *d_lmin = nullptr, *d_lmax = nullptr;
   bool have_moments = false;
@@ -267,18 +268,23 @@ void fill_node_args(sqb_ctx *c, NodeArgs &a) {
   a.stage_bytes = node_kernel_stage_bytes(c->n, c->stage_elems);
 }
 
-// Launch the node kernel over `count` nodes of d_list; returns SQB status.
-int run_nodes(sqb_ctx *c, NodeArgs &a, const int *d_list, int count) {
-  const int cols = choose_cols(c);
-  const int threads = node_kernel_threads(c->n, cols);
+// Layout, grid and scratch of a node-kernel launch over up to `count` nodes.
+int prepare_nodes(sqb_ctx *c, NodeArgs &a, int count, int *cols, int *grid) {
+  *cols = choose_cols(c);
+  const int threads = node_kernel_threads(c->n, *cols);
   if (threads > 1024) return SQB_ERR_UNSUPPORTED;
-  int grid = c->sms * (c->ctas_per_sm > 0 ? c->ctas_per_sm : 1);
-  if (grid > count) grid = count;
-  if (grid < 1) grid = 1;
-  int rc = ensure_scratch(c, grid);
-  if (rc) return rc;
+  *grid = std::max(1, std::min(c->sms * (c->ctas_per_sm > 0 ? c->ctas_per_sm : 1), count));
+  const int rc = ensure_scratch(c, *grid);
   a.scratch = c->d_scratch;
   a.scratch_stride = c->scratch_stride;
+  return rc;
+}
+
+// Launch the node kernel over `count` nodes of d_list; returns SQB status.
+int run_nodes(sqb_ctx *c, NodeArgs &a, const int *d_list, int count) {
+  int cols = 0, grid = 0;
+  const int rc = prepare_nodes(c, a, count, &cols, &grid);
+  if (rc) return rc;
   a.node_list = d_list;
   a.n_list = count;
   CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
@@ -425,7 +431,7 @@ int ensure_layers(sqb_ctx *c) {
   return SQB_OK;
 }
 
-// Whether the nonlocal forces of this context run on the sweep kernel.
+// Whether the SQ node work and the forces of this context run on the sweep kernel.
 int use_sweep(sqb_ctx *c, bool *yes) {
   *yes = false;
   if (c->node_kernel == SQB_KERNEL_PLANE) return SQB_OK;
@@ -433,27 +439,6 @@ int use_sweep(sqb_ctx *c, bool *yes) {
   if (rc) return rc;
   if (c->lay_state != 1) return c->node_kernel == SQB_KERNEL_SWEEP ? SQB_ERR_UNSUPPORTED : SQB_OK;
   *yes = true;
-  return SQB_OK;
-}
-
-// Kernel of the SQ node work: the plane-streaming kernel, the sweep kernel, or
-// its one-column tile.  The sweep kernel runs wherever it covers the context
-// but for the FP64 form with several projectors per slot, whose long Lanczos
-// runs end at a bound that follows the order of the sums (sqb_sweep_cols.cu):
-// that form keeps the kernel its results have always come from, the one-column
-// tile under first-fit layers and else the plane-streaming kernel, unless
-// SQB_KERNEL_SWEEP is asked for.
-enum class SqKernel { Plane, Sweep, Columns };
-int sq_kernel(sqb_ctx *c, bool fp64, SqKernel *k) {
-  bool sw = false;
-  const int rc = use_sweep(c, &sw);
-  if (rc) return rc;
-  *k = sw ? SqKernel::Sweep : SqKernel::Plane;
-  if (!sw || !fp64 || c->lay_pmax == 1) return SQB_OK;
-  int optin = 0;
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  if (c->lay_first_fit && sweep_cols_supported(c->n, c->n_gproj, 2, (size_t)optin)) *k = SqKernel::Columns;
-  else if (c->node_kernel != SQB_KERNEL_SWEEP) *k = SqKernel::Plane;
   return SQB_OK;
 }
 
@@ -526,54 +511,101 @@ int sweep_grid(sqb_ctx *c, int per_sm, SweepArgs &s, int *grid) {
   return rc;
 }
 
-// Window rows per thread of the one-column tile: three where asked for and covered, else two.
-int column_rows(const sqb_ctx *c) {
-  int optin = 0;
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  return c->sweep_ry == 3 && sweep_cols_supported(c->n, c->n_gproj, 3, (size_t)optin) ? 3 : 2;
-}
+// Lanczos steps, in window edges, up to which a node's bounds do not depend on
+// the order of the sums.  A Lanczos run keeps its vectors orthogonal until its
+// largest Ritz value has converged to rounding (Paige 1980), after about as
+// many steps as the spectral range, and so the window edge, asks for; from then
+// on rounding errors grow with every step and reach the smallest Ritz value.
+// Two kernels' bounds of LiH nodes (11^3 to 33^3 windows, 10 to 20 points per
+// cell, 34,000 nodes) agree to 1e-13 of the range up to 6.3 edges, to 1e-10 up
+// to 6.7, and beyond differ by up to the stop (1e-8 to 5e-7).  Al stops after
+// 1.6 to 2.7.
+constexpr int LANCZOS_STABLE_EDGES = 6;
 
-// Arguments, grid and scratch of an SQ launch on the sweep kernel (cols: its
-// one-column tile).
-int prepare_sq_sweep(sqb_ctx *c, const NodeArgs &a, bool cols, const int *d_list, int count, SweepArgs &s, int *grid) {
-  fill_sweep_args(c, d_list, count, s);
-  s.form = a.lq ? 2 : (a.mixed ? 1 : 0);
-  int per_sm = 0;
-  if (cols) {
-    s.ry = column_rows(c);
-    s.nsweep = sweep_cols_threads(c->n, s.ry);
-    CK(sweep_cols_per_sm(s, &per_sm));
-  } else {
-    CK(sweep_per_sm(s, &per_sm));
+// An SQ launch on the sweep kernel, and the launch behind it that repeats the
+// nodes with long Lanczos runs.  With several projectors per slot, where such
+// runs are met, those nodes keep the order of sums their bounds have always
+// come from: the one-column tile's under first-fit layers, else the
+// plane-streaming kernel's.
+enum class Redo { None, Columns, Plane };
+struct SqLaunch {
+  SweepArgs s, cols;
+  NodeArgs plane;
+  Redo redo = Redo::None;
+  int grid = 0, redo_grid = 0, layout = 0;
+};
+
+// Arguments, grids and scratch of an SQ launch on the sweep kernel.
+int prepare_sq_sweep(sqb_ctx *c, const NodeArgs &a, const int *d_list, int count, SqLaunch &l) {
+  fill_sweep_args(c, d_list, count, l.s);
+  l.s.form = a.lq ? 2 : (a.mixed ? 1 : 0);
+  l.s.lanczos_tol = a.lanczos_tol;
+  l.s.lz_chk = a.lz_chk;
+  l.s.chi = a.chi;
+  l.s.zee = a.zee;
+  l.s.rho_pj = a.rho_pj;
+  l.s.lmin = a.lmin;
+  l.s.lmax = a.lmax;
+  l.s.lanczos_iters = a.lanczos_iters;
+  if (l.s.form == 0 && c->lay_pmax > 1) {
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+    auto fits = [&](int ry) { return sweep_cols_supported(c->n, c->n_gproj, ry, (size_t)optin); };
+    l.redo = c->lay_first_fit && fits(2) ? Redo::Columns : Redo::Plane;
+    if (c->redo_n < count) {  // (a caller's list may name a node more than once)
+      c->redo_n = 0;
+      drop_graph(c);  // captured launches hold the old list's address
+      CK(dalloc(&c->d_redo, (size_t)count + 2));  // count, queue head, ids
+      c->redo_n = count;
+    }
+    l.cols = l.s;
+    l.cols.ry = c->sweep_ry == 3 && fits(3) ? 3 : 2;
+    l.cols.nsweep = sweep_cols_threads(c->n, l.cols.ry);
+    l.plane = a;
+    l.cols.node_list = l.plane.node_list = c->d_redo + 2;
+    l.cols.n_list_dev = l.plane.n_list_dev = c->d_redo;
+    l.cols.counter = l.plane.counter = c->d_redo + 1;
+    l.s.redo_count = c->d_redo;
+    l.s.redo_list = c->d_redo + 2;
+    l.s.redo_at = LANCZOS_STABLE_EDGES * c->n;
   }
-  return sweep_grid(c, per_sm, s, grid);
+  for (int pass = 0; pass < 2; pass++) {  // the second pass finds the scratch as large as both launches need
+    int per_sm = 0;
+    CK(sweep_per_sm(l.s, &per_sm));
+    int rc = sweep_grid(c, per_sm, l.s, &l.grid);
+    if (rc) return rc;
+    if (l.redo == Redo::Columns) {
+      CK(sweep_cols_per_sm(l.cols, &per_sm));
+      rc = sweep_grid(c, per_sm, l.cols, &l.redo_grid);
+    } else if (l.redo == Redo::Plane) {
+      rc = prepare_nodes(c, l.plane, count, &l.layout, &l.redo_grid);
+    }
+    if (rc) return rc;
+  }
+  return SQB_OK;
 }
 
 // Lanczos bounds and Chebyshev moments (MODE_SQ) of `count` nodes of d_list
 // with the outputs of `a`, on the sweep kernel where it covers the context,
 // else on the plane-streaming node kernel.
 int run_sq_nodes(sqb_ctx *c, NodeArgs &a, const int *d_list, int count) {
-  SqKernel k{};
-  int rc = sq_kernel(c, !a.mixed && !a.lq, &k);
+  bool sw = false;
+  int rc = use_sweep(c, &sw);
   if (rc) return rc;
-  c->stats.node_kernel = k == SqKernel::Plane ? SQB_KERNEL_PLANE : SQB_KERNEL_SWEEP;
-  if (k == SqKernel::Plane) return run_nodes(c, a, d_list, count);
-  SweepArgs s;
-  int grid = 0;
-  rc = prepare_sq_sweep(c, a, k == SqKernel::Columns, d_list, count, s, &grid);
+  c->stats.node_kernel = sw ? SQB_KERNEL_SWEEP : SQB_KERNEL_PLANE;
+  if (!sw) return run_nodes(c, a, d_list, count);
+  SqLaunch l;
+  rc = prepare_sq_sweep(c, a, d_list, count, l);
   if (rc) return rc;
-  s.lanczos_tol = a.lanczos_tol;
-  s.lz_chk = a.lz_chk;
-  s.chi = a.chi;
-  s.zee = a.zee;
-  s.rho_pj = a.rho_pj;
-  s.lmin = a.lmin;
-  s.lmax = a.lmax;
-  s.lanczos_iters = a.lanczos_iters;
   CK(cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
   CK(cudaMemsetAsync(c->d_proj_points, 0, 3 * sizeof(unsigned long long), c->stream));
-  CK(k == SqKernel::Columns ? launch_sweep_cols(s, grid, c->stream) : launch_sweep(s, grid, c->stream));
+  if (l.redo != Redo::None) CK(cudaMemsetAsync(c->d_redo, 0, 2 * sizeof(int), c->stream));
+  CK(launch_sweep(l.s, l.grid, c->stream));
+  if (l.redo == Redo::None) return SQB_OK;
+  CK(l.redo == Redo::Columns ? launch_sweep_cols(l.cols, l.redo_grid, c->stream)
+                             : launch_node_kernel(l.plane, l.redo_grid, l.layout, c->stream));
+  c->stats.kernel_launches += 1;
   return SQB_OK;
 }
 
@@ -872,7 +904,7 @@ int sqb_destroy(sqb_ctx *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   void *ptrs[] = {c->d_lay_id, c->d_lay_chi, c->d_rep_box, c->d_rep_gpb, c->d_rep_atom_l, c->d_rep_off_l, c->d_veff64, c->d_veffp, c->d_rep_nn, c->d_rep_atom, c->d_rep_off, c->d_typ_tab,
                   c->d_typ_nlocc, c->d_typ_nproj, c->d_typ_lmax, c->d_typ_lloc, c->d_typ_size, c->d_proj_denom,
-                  c->d_tables, c->d_rep_xyz, c->d_rep_off_ref, c->d_vjp, c->d_vjp_at, c->d_dtab, c->d_tab64, c->d_scratch, c->d_counter, c->d_nodes,
+                  c->d_tables, c->d_rep_xyz, c->d_rep_off_ref, c->d_vjp, c->d_vjp_at, c->d_dtab, c->d_tab64, c->d_scratch, c->d_counter, c->d_redo, c->d_nodes,
                   c->d_status, c->d_iters, c->d_proj_points, c->d_chi, c->d_zee, c->d_rho_pj, c->d_lmin,
                   c->d_lmax, c->d_xk, c->d_ctab, c->d_partial, c->d_result, c->d_rho, c->d_ci, c->d_fslots,
                   c->d_f, c->d_tmp, c->d_sens, c->d_loss, c->d_fermi, c->d_loc_type, c->d_loc_atom,
@@ -1478,11 +1510,8 @@ static int build_step_graph(sqb_ctx *c) {
   a.lmax = c->d_lmax;
   a.lanczos_iters = c->d_iters;
   {  // allocate what the captured launches use (no allocation inside a capture)
-    SqKernel k{};
-    SweepArgs s;
-    int grid = 0;
-    int rc0 = sq_kernel(c, !a.mixed && !a.lq, &k);
-    if (!rc0) rc0 = prepare_sq_sweep(c, a, k == SqKernel::Columns, c->d_nodes, c->nnode, s, &grid);
+    SqLaunch l;
+    const int rc0 = prepare_sq_sweep(c, a, c->d_nodes, c->nnode, l);
     if (rc0) return rc0;
   }
   FermiArgs fa = fermi_args(c);
@@ -1608,10 +1637,10 @@ static int spectral_quadrature(sqb_ctx *c, int scf_iter, double *lambda_f, doubl
   const double tol_eff = std::max(c->g.lanczos_tol, c->mixed_lanczos_tol);
   const bool defect = c->precision != SQB_FP64 && c->defect_budget > 0.0 && tol_eff > c->g.lanczos_tol;
   if (c->use_graph == 2 && !c->allreduce && !defect && c->have_veff && c->have_atoms && c->have_proj) {
-    SqKernel k{};
-    int rc0 = sq_kernel(c, c->precision == SQB_FP64, &k);
+    bool sw = false;
+    int rc0 = use_sweep(c, &sw);
     if (rc0) return rc0;
-    if (k != SqKernel::Plane) return run_step_graph(c, scf_iter, *lambda_f, lambda_f, rho, rho_pj, ci, chi, zee, ebs, eent);
+    if (sw) return run_step_graph(c, scf_iter, *lambda_f, lambda_f, rho, rho_pj, ci, chi, zee, ebs, eent);
   }
   int rc = sqb_lanczos_moments(c, chi, zee, rho_pj, nullptr, nullptr, nullptr);
   if (rc) return rc;
@@ -1731,10 +1760,10 @@ int sqb_autotune_sweep(sqb_ctx *c, int sample, int *rows, double *ms_out) {
   if (!c || sample < 0) return SQB_ERR_ARG;
   if (!c->have_veff || !c->have_atoms || !c->have_proj) return SQB_ERR_STATE;
   cudaSetDevice(c->device);
-  SqKernel kernel{};
-  int rc = sq_kernel(c, c->precision == SQB_FP64, &kernel);
+  bool sw = false;
+  int rc = use_sweep(c, &sw);
   if (rc) return rc;
-  if (kernel == SqKernel::Plane) return SQB_ERR_UNSUPPORTED;
+  if (!sw) return SQB_ERR_UNSUPPORTED;
   const int N = c->nnode;
   int count = sample > 0 ? sample : 2 * c->sms;
   if (count > N) count = N;
@@ -1749,8 +1778,7 @@ int sqb_autotune_sweep(sqb_ctx *c, int sample, int *rows, double *ms_out) {
   int best = 0;
   for (int k = 0; k < 2; k++) {
     c->sweep_ry = 2 + k;
-    if (c->sweep_ry == 3 && (kernel == SqKernel::Columns ? column_rows(c) : sweep_rows(c)) != 3)
-      continue;  // not covered for this window
+    if (c->sweep_ry == 3 && sweep_rows(c) != 3) continue;  // not covered for this window
     NodeArgs a;
     fill_node_args(c, a);
     a.mode = MODE_SQ;

@@ -79,6 +79,7 @@ struct NodeArgs {
   DevAtoms at;
   const int *node_list; // nodes to process
   int n_list;
+  const int *n_list_dev;  // their count on the device, or null
   int *counter;         // work-queue head (zeroed before launch)
   unsigned char *scratch;
   size_t scratch_stride; // bytes per CTA
@@ -155,8 +156,13 @@ struct SweepArgs {
   // work queue and outputs (indexed by node id)
   const int *node_list;
   int n_list;
+  const int *n_list_dev;  // their count on the device, or null: n_list
   int *counter;
   int *status;
+  // nodes whose Lanczos run has not stopped after redo_at steps are left to
+  // another kernel: their count, then their ids (null: none are)
+  int *redo_count, *redo_list;
+  int redo_at;
   unsigned char *scratch;
   size_t scratch_stride;  // bytes per CTA: three window vectors (FP64), then the flush buffer
   int nsweep;             // threads of the block (a multiple of 32)

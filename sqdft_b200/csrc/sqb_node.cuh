@@ -1987,7 +1987,7 @@ __global__ void __launch_bounds__(MAXT, 1) node_kernel(NodeArgs a) {
     if (threadIdx.x == 0) {
       const int q = atomicAdd(a.counter, 1);
       S.qidx = q;
-      S.node = q < a.n_list ? a.node_list[q] : -1;
+      S.node = q < (a.n_list_dev ? *a.n_list_dev : a.n_list) ? a.node_list[q] : -1;
       if (S.node >= 0) {
         S.gi = S.node % a.np[0];
         S.gj = (S.node / a.np[0]) % a.np[1];

@@ -1021,6 +1021,8 @@ static __device__ void start_vector(const SweepArgs &a, Shared &S, T *v, double 
   __syncthreads();
 }
 
+constexpr int LANCZOS_LEFT = 2;  // S.stop of a run left to another kernel (redo_at)
+
 // Lanczos bounds (sq.cpp:965-1092) in storage precision T, or (LQ) bounds and
 // moments from one FP64 Lanczos run started at e_c.  Sweep m applies H to the
 // unnormalised W_m = w_m-1 (v_m = s_m W_m), formed while it is loaded from the
@@ -1122,6 +1124,9 @@ __device__ void lanczos(const SweepArgs &a, Shared &S, unsigned char *dyn, doubl
         } else {
           S.count = m;  // the reference's count after this step
           S.stop = conv || S.count >= LANCZOS_MAX_ITER;
+          if constexpr (Tile::PM > 1 && std::is_same<T, double>::value) {
+            if (!S.stop && a.redo_count && m >= a.redo_at) S.stop = LANCZOS_LEFT;
+          }
         }
         if (S.count >= LANCZOS_MAX_ITER) atomicOr(a.status, ST_LANCZOS_MAXITER);
       }
@@ -1443,6 +1448,13 @@ __global__ void __launch_bounds__(MAXT, MINB) sweep_kernel(SweepArgs a) {
       using TL = typename std::conditional<FORM == 1, float, double>::type;
       if (FORM == 1) zero_planes(a, dyn, RY);  // FP32 values next
       lanczos<Tile, TL, false>(a, S, dyn, pcur, lmin, lmax, rows);
+      if constexpr (FORM == 0 && PM > 1) {
+        if (S.stop == LANCZOS_LEFT) {
+          if (threadIdx.x == 0) a.redo_list[atomicAdd(a.redo_count, 1)] = node;
+          __syncthreads();
+          continue;
+        }
+      }
       const double chi = (lmax + lmin) / 2, zee = (lmax - lmin) / 2;  // sq.cpp:564-565
       count_proj_points(a, S, rows + 1, 0);
       // moments stay FP64 in both forms: FP32 storage of the Chebyshev vectors

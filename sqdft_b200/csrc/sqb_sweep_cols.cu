@@ -1,19 +1,20 @@
-// Sweep kernel with one window column per thread: the FP64 SQ step of systems
-// with up to three projectors per ball.
+// Sweep kernel with one window column per thread: the nodes of systems with up
+// to three projectors per ball whose FP64 Lanczos runs are long.
 //
-// Their Lanczos runs are long (LiH at h = 0.386, 33^3 windows: 106 to 290
-// steps, where Al needs about 60) and the stop is reached on a plateau of the
-// smallest eigenvalue, so at some nodes the accepted bound depends on the
-// rounding of every sum before it: relative noise of 1e-16 on the vectors of a
-// plain FP64 Lanczos run moves it by up to 1e-6 Ha, the stop itself, and the
-// moments of the block by 2e-7.  No order of the sums is better than another
-// there, but a caller's results should not change with the tile the kernel
-// happens to use, so this step keeps the sums it always had: this kernel where
-// first-fit layers cover the system, the plane-streaming kernel where they do
-// not.  The pairs of columns of sqb_sweep.cuh do the same step in another
-// order 1.1 to 3.5 times faster (64-atom LiH, 400 nodes of 33^3 windows: 192 ms
-// against 665 on the plane-streaming kernel); SQB_KERNEL_SWEEP asks for them
-// where only they cover the system.
+// A run past about 6.5 window edges has lost the orthogonality of its vectors
+// (LiH at h = 0.386, 33^3 windows: 87 to 290 steps, one node in ten past 198).
+// Where it stops on a plateau of the smallest eigenvalue, the accepted bound
+// then depends on the rounding of every sum before it: relative noise of 1e-16
+// on the vectors of a plain FP64 run with exact projections moves it by up to
+// 1e-6 Ha, the stop itself, and the moments of the block by 2e-7.  No order of
+// the sums is better than another there, but a caller's results should not
+// change with the tile that is fastest.  So the column-pair kernel
+// (sqb_sweep.cuh) leaves such nodes to a second launch, whose sums keep the
+// order these bounds have always come from: of this kernel where first-fit
+// layers cover the system, of the plane-streaming kernel where they do not.
+// Measured on the B200, FP64 step: 64-atom LiH, 400 nodes of 33^3 windows,
+// 736 ms all on the plane-streaming kernel, 538 with its long runs there (145
+// to 240 on column pairs alone).
 //
 // The plane loop is that of sqb_sweep.cuh without the pairs: window vectors of
 // n^3 values, a thread per column and RY adjacent rows, the stencil's planes
@@ -394,7 +395,7 @@ __global__ void __launch_bounds__(MAXT, 1) sweep_cols_kernel(SweepArgs a) {
     if (threadIdx.x == 0) {
       const int q = atomicAdd(a.counter, 1);
       S.qidx = q;
-      S.node = q < a.n_list ? a.node_list[q] : -1;
+      S.node = q < (a.n_list_dev ? *a.n_list_dev : a.n_list) ? a.node_list[q] : -1;
       if (S.node >= 0) {
         S.gi = S.node % a.np[0];
         S.gj = (S.node / a.np[0]) % a.np[1];

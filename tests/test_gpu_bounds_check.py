@@ -32,6 +32,7 @@ import json, sys
 import numpy as np
 sys.path.insert(0, sys.argv[1])
 from perf import cases
+from sqdft_b200 import sq
 
 out = {}
 for system in ("al", "lih"):
@@ -47,6 +48,17 @@ for system in ("al", "lih"):
                 r = (r["chi"], r["zee"])
             r = [float(np.abs(x).sum()) for x in (r if isinstance(r, tuple) else (r,))]
             out[f"{system}-{nloc}-{rows}-{kind}"] = dict(kernel=kernel, **{str(i): x for i, x in enumerate(r)})
+for nloc, rows in ((10, 0), (16, 0), (14, 3)):  # long Lanczos runs: the one-column tile
+    c = cases._case(dict(kind="sq", system="lih", form=0, cells=1, per_cell=20, block="3x2x2", nloc=nloc, npl=20,
+                         kt=9.0), 3)
+    c.lanczos_tol = 1e-12
+    with sq.Context(c, precision=0) as ctx:
+        ctx.nonlocal_projectors()
+        ctx.set_veff(c.veff)
+        ctx.set_sweep_rows(rows)
+        r = ctx.lanczos_moments()
+        assert (r["lanczos_iters"] > 6 * c.nw).any()
+        out[f"long-{nloc}-{rows}"] = dict(kernel=ctx.stats()["node_kernel"], chi=float(np.abs(r["chi"]).sum()))
 print("RESULT " + json.dumps(out))
 """
 
@@ -105,7 +117,7 @@ def test_bounds_check_build_runs_clean_and_agrees():
 
 
 def test_bounds_check_of_synthetic_systems():
-    """The tiles (one column, pairs, three rows) and the adjoint, many nodes per CTA among them."""
+    """The tiles (pairs, three rows, one column) and the adjoint, many nodes per CTA among them."""
     assert BC_LIB.exists(), f"bounds-check library not built: {BC_LIB}"
     checked = _run(BC_LIB, SYNTHETIC)
     normal = _run(None, SYNTHETIC)
