@@ -192,13 +192,15 @@ int sqb_set_launch(sqb_ctx *ctx, int ctas_per_sm, int cols_per_thread);
 #define SQB_KERNEL_PLANE 1
 #define SQB_KERNEL_SWEEP 2
 int sqb_set_node_kernel(sqb_ctx *ctx, int kernel);
-/* Tile of the sweep kernel's threads: 0 or 2 the default one (a pair of window
- * columns and one row per thread), 3 a pair of columns and three rows (fewer
- * threads, more registers each; windows up to 33 wide).  Results agree to
- * rounding (the block reductions sum in another order). */
+/* Window rows per thread of the sweep kernel's one-column tile, which the FP64
+ * step of systems with more than one projector per ball repeats nodes with
+ * long Lanczos runs on: 2 (0: the same) or 3 (windows up to 33 wide, else
+ * SQB_ERR_UNSUPPORTED).  Results agree to rounding (the block reductions sum in
+ * another order).  All other sweeps run one tile, a pair of window columns and
+ * one row per thread, whatever is asked for here. */
 int sqb_set_sweep_rows(sqb_ctx *ctx, int rows);
-/* Times the SQ node work on the sweep kernel with the default tile (2) and
- * with three rows per thread (3) on `sample` evenly spaced nodes (0: two per SM), keeps the
+/* Times the SQ node work on the sweep kernel with two and with three rows per
+ * thread (above) on `sample` evenly spaced nodes (0: two per SM), keeps the
  * faster for the context; *rows the choice, ms[2] the times (-1 where a
  * variant does not apply).  SQB_ERR_UNSUPPORTED when the sweep kernel does
  * not cover the context. */

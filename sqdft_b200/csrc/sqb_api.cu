@@ -71,7 +71,7 @@ struct sqb_ctx {
   // Sweep kernel (sqb_sweep.cuh) and its layered projector fields, built on
   // first use after the projector tables are set.
   int node_kernel = SQB_KERNEL_AUTO;
-  int sweep_ry = 0;  // window rows per sweep-kernel thread (0: automatic)
+  int sweep_ry = 0;  // window rows per thread of the one-column tile (0: two)
   int lay_state = 0;  // 0 not built, 1 built and usable, -1 the sweep kernel does not cover this context
   bool lay_first_fit = false;  // the layers are those of first fit in replica order
   int n_gproj = 0, lay_pmax = 1, n_lrep = 0;
@@ -394,7 +394,7 @@ int ensure_layers(sqb_ctx *c) {
   const long long evol = (long long)c->exp * c->ey * c->ez;
   const bool usable = n_layers <= LAYERS && pmax <= LAY_PMAX && ngp + pm < 65535 &&
                       evol * LAYERS * LAY_PMAX < (1LL << 31) &&
-                      sweep_rows_supported(c->n, 1) && sweep_smem(c->n, pm, ngp, 1) <= (size_t)optin &&
+                      sweep_window_supported(c->n) && sweep_smem(c->n, pm, ngp) <= (size_t)optin &&
                       c->n_typ < 256;
   if (!usable) return SQB_OK;
   c->lay_first_fit = first_fit;
@@ -456,17 +456,6 @@ int ensure_sweep_scratch(sqb_ctx *c, int grid, size_t *stride) {
   return SQB_OK;
 }
 
-// Window rows per sweep-kernel thread: three where asked for (sqb_set_sweep_rows,
-// sqb_autotune_sweep) and covered, else the default tile's.
-int sweep_rows(const sqb_ctx *c) {
-  int optin = 0;
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  if (c->sweep_ry == 3 && sweep_rows_supported(c->n, 3) &&
-      sweep_smem(c->n, c->lay_pmax, c->n_gproj, 3) <= (size_t)optin)
-    return 3;
-  return 1;
-}
-
 // The context's part of a sweep-kernel launch (grid, fields, replicas, queue).
 void fill_sweep_args(sqb_ctx *c, const int *d_list, int count, SweepArgs &s) {
   std::memset(&s, 0, sizeof(s));
@@ -496,8 +485,7 @@ void fill_sweep_args(sqb_ctx *c, const int *d_list, int count, SweepArgs &s) {
   s.n_list = count;
   s.counter = c->d_counter;
   s.status = c->d_status;
-  s.ry = sweep_rows(c);
-  s.nsweep = sweep_threads(c->n, s.ry);
+  s.nsweep = sweep_threads(c->n);
   s.proj_points = c->d_proj_points;
 }
 
@@ -1661,7 +1649,7 @@ static int spectral_quadrature(sqb_ctx *c, int scf_iter, double *lambda_f, doubl
 
 int sqb_set_sweep_rows(sqb_ctx *c, int rows) {
   if (!c || (rows != 0 && rows != 2 && rows != 3)) return SQB_ERR_ARG;
-  if (rows == 3 && !sweep_rows_supported(c->n, 3)) return SQB_ERR_UNSUPPORTED;
+  if (rows == 3 && !sweep_cols_supported(c->n, 0, 3, ~size_t(0))) return SQB_ERR_UNSUPPORTED;
   c->sweep_ry = rows;
   drop_graph(c);
   return SQB_OK;
@@ -1778,7 +1766,7 @@ int sqb_autotune_sweep(sqb_ctx *c, int sample, int *rows, double *ms_out) {
   int best = 0;
   for (int k = 0; k < 2; k++) {
     c->sweep_ry = 2 + k;
-    if (c->sweep_ry == 3 && sweep_rows(c) != 3) continue;  // not covered for this window
+    if (c->sweep_ry == 3 && !sweep_cols_supported(c->n, 0, 3, ~size_t(0))) continue;  // not covered for this window
     NodeArgs a;
     fill_node_args(c, a);
     a.mode = MODE_SQ;

@@ -39,34 +39,33 @@ __global__ void fill_empty_kernel(unsigned long long *lay_id, long long evol, un
 
 template <int PM, int FORM>
 struct SqKernels {
-  template <int MAXT, int RY, int MINB>
+  template <int MAXT, int MINB>
   static const void *get() {
-    return reinterpret_cast<const void *>(&sweep::sweep_kernel<PM, FORM, MAXT, RY, MINB>);
+    return reinterpret_cast<const void *>(&sweep::sweep_kernel<PM, FORM, MAXT, sweep::TILE_RY, MINB>);
   }
 };
 
 const void *sq_kernel(const SweepArgs &a) {
   if (a.pmax == 1)
-    return a.form == 0   ? sweep::pick_tile<SqKernels<1, 0>>(a.n, a.ry)
-           : a.form == 1 ? sweep::pick_tile<SqKernels<1, 1>>(a.n, a.ry)
-                         : sweep::pick_tile<SqKernels<1, 2>>(a.n, a.ry);
+    return a.form == 0   ? sweep::pick_tile<SqKernels<1, 0>>(a.n)
+           : a.form == 1 ? sweep::pick_tile<SqKernels<1, 1>>(a.n)
+                         : sweep::pick_tile<SqKernels<1, 2>>(a.n);
   if (a.pmax == 3)
-    return a.form == 0   ? sweep::pick_tile<SqKernels<3, 0>>(a.n, a.ry)
-           : a.form == 1 ? sweep::pick_tile<SqKernels<3, 1>>(a.n, a.ry)
-                         : sweep::pick_tile<SqKernels<3, 2>>(a.n, a.ry);
+    return a.form == 0   ? sweep::pick_tile<SqKernels<3, 0>>(a.n)
+           : a.form == 1 ? sweep::pick_tile<SqKernels<3, 1>>(a.n)
+                         : sweep::pick_tile<SqKernels<3, 2>>(a.n);
   return nullptr;
 }
 
 }  // namespace
 
-int sweep_threads(int n, int ry) { return sweep::sweep_threads_of(n, ry); }
+int sweep_threads(int n) { return sweep::sweep_threads_of(n, sweep::TILE_RY); }
 
-bool sweep_rows_supported(int n, int ry) {
-  return (ry == 1 && n <= sweep::TILE_N_MAX) || (ry == 3 && n <= sweep::TILE_N_ROWS3);
-}
+bool sweep_window_supported(int n) { return n <= sweep::TILE_N_MAX; }
 
-size_t sweep_smem(int n, int pmax, int n_gproj, int ry) {
-  return sweep::shared_fixed() + sweep::planes_bytes(n, ry) + sweep::ring_bytes(sweep::tile_bound(n, ry), ry) +
+size_t sweep_smem(int n, int pmax, int n_gproj) {
+  return sweep::shared_fixed() + sweep::planes_bytes(n, sweep::TILE_RY) +
+         sweep::ring_bytes(sweep::tile_bound(n), sweep::TILE_RY) +
          (((size_t)(n_gproj + pmax) * sizeof(double) + 127) & ~size_t(127));
 }
 
@@ -92,8 +91,8 @@ cudaError_t kernel_setup(const void *kernel, int threads, size_t smem, int *per_
 }
 
 cudaError_t tile_setup(const void *kernel, const SweepArgs &a, int *per_sm) {
-  if (a.n > MAXN || sweep_threads_of(a.n, a.ry) != a.nsweep) return cudaErrorInvalidConfiguration;
-  return kernel_setup(kernel, a.nsweep, sweep_smem(a.n, a.pmax, a.n_gproj, a.ry), per_sm);
+  if (a.n > MAXN || sweep_threads_of(a.n, TILE_RY) != a.nsweep) return cudaErrorInvalidConfiguration;
+  return kernel_setup(kernel, a.nsweep, sweep_smem(a.n, a.pmax, a.n_gproj), per_sm);
 }
 
 }  // namespace sweep
@@ -106,7 +105,7 @@ cudaError_t launch_sweep(const SweepArgs &a, int grid, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   SweepArgs args = a;
   void *argv[] = {&args};
-  return cudaLaunchKernel(kernel, dim3(grid), dim3(a.nsweep), argv, sweep_smem(a.n, a.pmax, a.n_gproj, a.ry), s);
+  return cudaLaunchKernel(kernel, dim3(grid), dim3(a.nsweep), argv, sweep_smem(a.n, a.pmax, a.n_gproj), s);
 }
 
 cudaError_t launch_fill_layers(int n_rep, const int4 *rep_box, const int *rep_gpb, const int *typ_nlocc,

@@ -1474,35 +1474,40 @@ __global__ void __launch_bounds__(MAXT, MINB) sweep_kernel(SweepArgs a) {
   }
 }
 
-// Tiles: rows per thread and the launch bound, which sets the registers per
-// thread.  One row per thread by default: two rows share their y-arm loads and
-// issue 20% fewer instructions per point, but their 8 warps of 255 registers
-// hide less latency than 16 warps of 128 (B200, 288 nodes of 31^3 windows,
-// FP64: 25.4 against 20.8 ms; 27^3: 23.4 against 16.6 ms; 39^3, 13 against 25
-// warps: the same).  The bounds follow the registers a warp count leaves (39^3:
-// 124.7 ms at a bound of 896 and 72 registers, 144.5 at 1024 and 64).  Windows
-// up to 19 wide keep two CTAs on an SM or more, but not at fewer registers:
-// three at 112 took 13.3 ms where two at 168 take 9.6 (17^3, 1000 nodes).
-constexpr int TILE_N_MAX = 43;    // widest window of the default tiles
-constexpr int TILE_N_ROWS3 = 33;  // and of three rows per thread
+// Tiles: a pair of columns and one row per thread, and a launch bound, which
+// sets the registers per thread.  More rows share their y-arm loads and issue
+// 20% fewer instructions per point, but leave fewer warps to hide latency.  Two
+// rows, 8 warps of 255 registers against 16 of 128 (B200, 288 nodes of 31^3
+// windows, FP64): 25.4 against 20.8 ms; 27^3: 23.4 against 16.6 ms.  Three rows
+// (448 nodes, npl 64, FP64 step of Al): 7.5 against 1.6 ms at 9^3, 32 against 12
+// at 21^3, 76 against 31 at 31^3, 94 against 55 at 33^3, and 1.4 to 10 times
+// longer in the other forms, the forces, the adjoint and LiH.  The bounds follow
+// the registers a warp count leaves (39^3: 124.7 ms at a bound of 896 and 72
+// registers, 144.5 at 1024 and 64).  Shared memory holds three CTAs on an SM at
+// 9^3, two from 11^3 to 19^3 (17^3: 82 KB each); fewer registers for the same two
+// cost time (17^3, 1000 nodes: 13.3 ms at 112, 9.6 at 168).  From 23^3 on one CTA
+// keeps 168 registers: 14.6, 17.6 and 20.0 ms at 23^3, 25^3 and 27^3 (448 nodes
+// as above), against 24.4, 30.5 and 38.6 for two CTAs of 80.  The forces and the
+// adjoint take the same tiles.
+constexpr int TILE_RY = 1;
+constexpr int TILE_N_MAX = 43;  // widest window
 // Launch bound of the tile (and the ring's stride).
-inline int tile_bound(int n, int ry) {
-  const int t = sweep_threads_of(n, ry);
-  return ry == 3 ? 192 : t <= 64 ? 64 : t <= 192 ? 192 : t <= 384 ? 384 : t <= 512 ? 512 : t <= 640 ? 640 : t <= 768 ? 768 : t <= 896 ? 896 : 1024;
+inline int tile_bound(int n) {
+  const int t = sweep_threads_of(n, TILE_RY);
+  return t <= 64 ? 64 : t <= 192 ? 192 : t <= 384 ? 384 : t <= 512 ? 512 : t <= 640 ? 640 : t <= 768 ? 768 : t <= 896 ? 896 : 1024;
 }
 template <class K>
-const void *pick_tile(int n, int ry) {
-  if (ry == 3) return n <= TILE_N_ROWS3 ? K::template get<192, 3, 1>() : nullptr;
-  if (ry != 1 || n > TILE_N_MAX) return nullptr;
-  const int m = tile_bound(n, ry);
-  return m == 64    ? K::template get<64, 1, 4>()
-         : m == 192 ? K::template get<192, 1, 2>()
-         : m == 384 ? K::template get<384, 1, 1>()
-         : m == 512 ? K::template get<512, 1, 1>()
-         : m == 640 ? K::template get<640, 1, 1>()
-         : m == 768 ? K::template get<768, 1, 1>()
-         : m == 896 ? K::template get<896, 1, 1>()
-                    : K::template get<1024, 1, 1>();
+const void *pick_tile(int n) {
+  if (n > TILE_N_MAX) return nullptr;
+  const int m = tile_bound(n);
+  return m == 64    ? K::template get<64, 3>()
+         : m == 192 ? K::template get<192, 2>()
+         : m == 384 ? K::template get<384, 1>()
+         : m == 512 ? K::template get<512, 1>()
+         : m == 640 ? K::template get<640, 1>()
+         : m == 768 ? K::template get<768, 1>()
+         : m == 896 ? K::template get<896, 1>()
+                    : K::template get<1024, 1>();
 }
 // Shared-memory limit of a kernel for a launch and, on request, its resident
 // CTAs per SM; tile_setup: of a default-tile kernel for the launch `a`.

@@ -431,7 +431,7 @@ constexpr int COL_A = 512, COL_B = 576, COL_C = 1024, COL_R3 = 384;
 const void *cols_kernel(int n, int ry) {
   const int t = col_threads(n, ry);
   if (ry == 3) return t <= COL_R3 ? reinterpret_cast<const void *>(&sweep_cols_kernel<COL_R3, 3>) : nullptr;
-  if (ry != 2 || n > TILE_N_MAX) return nullptr;
+  if (ry != 2) return nullptr;
   return t <= COL_A   ? reinterpret_cast<const void *>(&sweep_cols_kernel<COL_A, 2>)
          : t <= COL_B ? reinterpret_cast<const void *>(&sweep_cols_kernel<COL_B, 2>)
          : t <= COL_C ? reinterpret_cast<const void *>(&sweep_cols_kernel<COL_C, 2>)

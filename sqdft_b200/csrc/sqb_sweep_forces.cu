@@ -8,19 +8,19 @@ namespace {
 
 template <int PM, typename T>
 struct ForceKernels {
-  template <int MAXT, int RY, int MINB>
+  template <int MAXT, int MINB>
   static const void *get() {
-    return reinterpret_cast<const void *>(&sweep::sweep_force_kernel<PM, T, MAXT, RY, MINB>);
+    return reinterpret_cast<const void *>(&sweep::sweep_force_kernel<PM, T, MAXT, sweep::TILE_RY, MINB>);
   }
 };
 
 const void *force_kernel(const SweepArgs &a, int single) {
   if (a.pmax == 1)
-    return single ? sweep::pick_tile<ForceKernels<1, float>>(a.n, a.ry)
-                  : sweep::pick_tile<ForceKernels<1, double>>(a.n, a.ry);
+    return single ? sweep::pick_tile<ForceKernels<1, float>>(a.n)
+                  : sweep::pick_tile<ForceKernels<1, double>>(a.n);
   if (a.pmax == 3)
-    return single ? sweep::pick_tile<ForceKernels<3, float>>(a.n, a.ry)
-                  : sweep::pick_tile<ForceKernels<3, double>>(a.n, a.ry);
+    return single ? sweep::pick_tile<ForceKernels<3, float>>(a.n)
+                  : sweep::pick_tile<ForceKernels<3, double>>(a.n);
   return nullptr;
 }
 
@@ -36,7 +36,7 @@ cudaError_t launch_sweep_forces(const SweepArgs &a, int single, int grid, cudaSt
   if (e != cudaSuccess) return e;
   SweepArgs args = a;
   void *argv[] = {&args};
-  return cudaLaunchKernel(kernel, dim3(grid), dim3(a.nsweep), argv, sweep_smem(a.n, a.pmax, a.n_gproj, a.ry), s);
+  return cudaLaunchKernel(kernel, dim3(grid), dim3(a.nsweep), argv, sweep_smem(a.n, a.pmax, a.n_gproj), s);
 }
 
 }  // namespace sqb

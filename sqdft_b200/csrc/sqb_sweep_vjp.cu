@@ -268,15 +268,15 @@ __global__ void __launch_bounds__(MAXT, MINB) sweep_vjp_kernel(SweepArgs a) {
 
 template <int PM>
 struct VjpKernels {
-  template <int MAXT, int RY, int MINB>
+  template <int MAXT, int MINB>
   static const void *get() {
-    return reinterpret_cast<const void *>(&sweep_vjp_kernel<PM, MAXT, RY, MINB>);
+    return reinterpret_cast<const void *>(&sweep_vjp_kernel<PM, MAXT, TILE_RY, MINB>);
   }
 };
 
 const void *vjp_kernel(const SweepArgs &a) {
-  return a.pmax == 1   ? pick_tile<VjpKernels<1>>(a.n, a.ry)
-         : a.pmax == 3 ? pick_tile<VjpKernels<3>>(a.n, a.ry)
+  return a.pmax == 1   ? pick_tile<VjpKernels<1>>(a.n)
+         : a.pmax == 3 ? pick_tile<VjpKernels<3>>(a.n)
                        : nullptr;
 }
 
@@ -295,7 +295,7 @@ cudaError_t launch_sweep_vjp(const SweepArgs &a, int grid, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   SweepArgs args = a;
   void *argv[] = {&args};
-  return cudaLaunchKernel(kernel, dim3(grid), dim3(a.nsweep), argv, sweep_smem(a.n, a.pmax, a.n_gproj, a.ry), s);
+  return cudaLaunchKernel(kernel, dim3(grid), dim3(a.nsweep), argv, sweep_smem(a.n, a.pmax, a.n_gproj), s);
 }
 
 }  // namespace sqb

@@ -255,11 +255,11 @@ class Context:
         _check(self.lib.sqb_set_veff(self.ptr, _d(v)), "sqb_set_veff")
 
     def set_sweep_rows(self, rows: int = 0):
-        """sqb_set_sweep_rows: tile of a sweep-kernel thread (0 or 2 the default, 3 three rows)."""
+        """sqb_set_sweep_rows: window rows per thread of the one-column tile (0 or 2, 3)."""
         _check(self.lib.sqb_set_sweep_rows(self.ptr, int(rows)), "sqb_set_sweep_rows")
 
     def autotune_sweep(self, sample: int = 0):
-        """sqb_autotune_sweep: (tile chosen, [ms with the default tile (2), ms with three rows (3)])."""
+        """sqb_autotune_sweep: (rows chosen, [ms with 2 rows, ms with 3 rows])."""
         rows = C.c_int()
         ms = np.zeros(2)
         _check(self.lib.sqb_autotune_sweep(self.ptr, int(sample), C.byref(rows), _d(ms)), "sqb_autotune_sweep")

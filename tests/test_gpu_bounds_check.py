@@ -117,7 +117,7 @@ def test_bounds_check_build_runs_clean_and_agrees():
 
 
 def test_bounds_check_of_synthetic_systems():
-    """The tiles (pairs, three rows, one column) and the adjoint, many nodes per CTA among them."""
+    """The tiles (pairs, one column of two and of three rows) and the adjoint, many nodes per CTA among them."""
     assert BC_LIB.exists(), f"bounds-check library not built: {BC_LIB}"
     checked = _run(BC_LIB, SYNTHETIC)
     normal = _run(None, SYNTHETIC)

@@ -67,11 +67,14 @@ def test_tiles_match_plane_kernel(system, nloc):
     _check_tiles(system, nloc)
 
 
-@pytest.mark.parametrize("system", ["al", "lih"])
-@pytest.mark.parametrize("nloc", [4, 8, 9, 16])
-def test_three_row_tiles_match_plane_kernel(system, nloc):
-    """Three rows per thread: edges 9, 17, 19 and 33, n mod 3 = 0, 2, 1 and the widest."""
-    _check_tiles(system, nloc, rows=3)
+@pytest.mark.parametrize("kind,form", [("sq", 0), ("sq", 1), ("sq", 2), ("forces", 0), ("forces", 1)])
+def test_sweep_rows_leave_the_pair_tile_alone(kind, form):
+    """Three rows per thread were up to seven times slower than the pair tile: rows = 3 is accepted
+    and runs it, to the bit, where no node runs on the one-column tile."""
+    a, _ = _both(_params(kind, "al", 9, form))
+    b, _ = _both(_params(kind, "al", 9, form), rows=3)
+    for x, y in zip(a.values(), b.values()) if kind == "sq" else [(a, b)]:
+        assert np.array_equal(x, y)
 
 
 @pytest.mark.parametrize("system", ["al", "lih"])
@@ -89,14 +92,6 @@ def test_many_nodes_per_cta(system):
 def test_adjoint_matches_plane_kernel(system, nloc, npl):
     """Block remainders of the quadratic form (16 vectors, 8 at a time), one block and several."""
     (gv, ga), (gv0, ga0) = _both(_params("vjp", system, nloc, npl=npl, per_cell=20))
-    assert _rel(gv, gv0) <= 1e-12
-    assert _rel(ga, ga0) <= 1e-11
-
-
-@pytest.mark.parametrize("system,nloc,npl", [("al", 4, 20), ("al", 8, 16), ("al", 9, 16), ("al", 16, 12),
-                                             ("lih", 4, 20), ("lih", 8, 16), ("lih", 9, 16), ("lih", 16, 12)])
-def test_three_row_adjoint_matches_plane_kernel(system, nloc, npl):
-    (gv, ga), (gv0, ga0) = _both(_params("vjp", system, nloc, npl=npl, per_cell=20), rows=3)
     assert _rel(gv, gv0) <= 1e-12
     assert _rel(ga, ga0) <= 1e-11
 
