@@ -387,7 +387,8 @@ def run_ours(args):
 
     peak, peak_kind = hbm_peak()
     # DRAM bytes per node matvec step of the node kernel, measured with ncu on
-    # a node sample of the configuration (profiles/sweep_kernel_c2_traffic.md)
+    # nodes of the configuration's windows, where they have been
+    # (profiles/sweep_kernel_c2_traffic.md)
     traffic = {}
     tr = ROOT / "profiles" / "sweep_kernel_traffic.json"
     if tr.exists():
@@ -680,7 +681,7 @@ def main():
     ap.add_argument("--sample-nodes", type=int, default=0,
                     help="time the node kernel alone on this many nodes (needs --precision fp64|mixed|lq)")
     ap.add_argument("--sweep-rows", type=int, default=0, choices=[0, 2, 3],
-                    help="window rows per sweep-kernel thread (0: the library's choice)")
+                    help="window rows per thread of the sweep kernel's one-column tile (0: the library's choice)")
     ap.add_argument("--forces-only", action="store_true",
                     help="one SQ step, then time ForcesNonLocal alone (needs --precision fp64|mixed)")
     ap.add_argument("--scf-steps", type=int, default=0,

@@ -356,8 +356,13 @@ int ensure_layers(sqb_ctx *c) {
     // their common neighbours then cannot share.  Colouring next the ball whose
     // neighbours already use the most layers (DSATUR, Brelaz 1979) finds the
     // four sublattices of a displaced FCC cell: of the 108-atom cell's blocks
-    // one in three failed by first fit, of 64-atom LiH every one, and then ran
-    // on the plane-streaming kernel at less than half the speed.
+    // one in three failed by first fit, of 64-atom LiH nearly every one, and
+    // then ran on the plane-streaming kernel at less than half the speed.  Al
+    // at 8 to 18 points per cell and LiH at 10, 12 and 14 to 20 have four
+    // layers (LiH at 16 once in four displacements five).  LiH at 11 and 13
+    // needs eight or nine, for any colouring: there a ball's box is as wide as
+    // the cell, displaced balls of one sublattice overlap, and the system stays
+    // on the plane-streaming kernel.
     std::fill(layer_of.begin(), layer_of.end(), -1);
     std::vector<std::vector<char>> seen(nb);  // layers among a ball's neighbours
     std::vector<int> sat(nb, 0);

@@ -36,8 +36,8 @@
 // (sq.cpp:965-1092) with one sweep per step: the sweep forms the next
 // unnormalised Lanczos vector from the stored vectors while loading it, and
 // the block then finds the extreme eigenvalues of the tridiagonal (the
-// quantities TridiagEigenSolve sq.cpp:1094-1180 returns) by a 257-way
-// multisection.  Chebyshev moments use the reference's doubling identities
+// quantities TridiagEigenSolve sq.cpp:1094-1180 returns) by a
+// (16 warps + 1)-way multisection (33-way on two warps, 481-way on thirty).  Chebyshev moments use the reference's doubling identities
 // (sq.cpp:564-655).  The Lanczos-quadrature form takes bounds and moments from
 // one Lanczos run started at the node (Gauss-quadrature identity).
 #include <cmath>
@@ -312,9 +312,9 @@ struct PairOf<float> {
 // behind in the thread's own slots of a shared ring.
 //
 // What bounds it is latency and instruction issue (B200, 31^3 windows, force
-// sweeps: 52% of issue slots, 65% inside the plane loop; 334 thread
-// instructions per point, 118 of them integer and 57 FP64), not FP64 (13% of
-// the pipe) and not memory (57 bytes per point, from L2).  A pair of columns
+// sweeps: 49% of issue slots; 298 thread instructions per point, 56 of them
+// FP64), not FP64 (17.5% of the pipe) and not memory (132 bytes per point
+// through L2, 37 of them to or from DRAM: 2.0 TB/s).  A pair of columns
 // per thread takes its x-arm values in 3 16-byte loads per point where a single
 // column takes 12 8-byte ones.  The streamed operands bypass L1 (__ldcg,
 // __stcg), which the shared memory leaves small, so that it keeps the spilled
