@@ -178,7 +178,7 @@ int sqb_set_launch(sqb_ctx *ctx, int ctas_per_sm, int cols_per_thread);
  * projectors per type.  SQB_KERNEL_PLANE: the plane-streaming kernel with
  * per-window box lists, any system.  SQB_KERNEL_AUTO (default): the sweep
  * kernel where it covers the system.  Results agree to rounding; a Lanczos run
- * of more than about 6.5 window edges (LiH; Al stops after 1.6 to 2.7)
+ * of more than about 6.5 window edges (LiH; Al stops after 1.6 to 2.6)
  * amplifies it, and its bounds can move by up to the stop with the order of
  * the sums.  In the FP64 step of systems with more than one projector per ball
  * the sweep kernel therefore repeats the nodes whose runs pass six edges in a

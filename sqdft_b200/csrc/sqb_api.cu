@@ -510,9 +510,10 @@ int sweep_grid(sqb_ctx *c, int per_sm, SweepArgs &s, int *grid) {
 // many steps as the spectral range, and so the window edge, asks for; from then
 // on rounding errors grow with every step and reach the smallest Ritz value.
 // Two kernels' bounds of LiH nodes (11^3 to 33^3 windows, 10 to 20 points per
-// cell, 34,000 nodes) agree to 1e-13 of the range up to 6.3 edges, to 1e-10 up
-// to 6.7, and beyond differ by up to the stop (1e-8 to 5e-7).  Al stops after
-// 1.6 to 2.7.
+// cell, 52,000 nodes) agree to 1e-15 of the range up to 5.7 edges, to 1e-13 up
+// to 6.3 and to 1e-10 up to 6.8, and from 7 on (of up to 12.5) they differ by up
+// to the stop (1e-8 to 5e-7).  One node in 28 passes six edges.  Al stops after
+// 1.6 to 2.6.
 constexpr int LANCZOS_STABLE_EDGES = 6;
 
 // An SQ launch on the sweep kernel, and the launch behind it that repeats the
