@@ -2,7 +2,7 @@
 // to three projectors per ball whose FP64 Lanczos runs are long.
 //
 // A run past about 6.5 window edges has lost the orthogonality of its vectors
-// (LiH at h = 0.386, 33^3 windows: 87 to 290 steps, one node in ten past 198).
+// (LiH at h = 0.386, 33^3 windows: 80 to 321 steps, one node in twelve past 198).
 // Where it stops on a plateau of the smallest eigenvalue, the accepted bound
 // then depends on the rounding of every sum before it: relative noise of 1e-16
 // on the vectors of a plain FP64 run with exact projections moves it by up to
@@ -12,9 +12,9 @@
 // (sqb_sweep.cuh) leaves such nodes to a second launch, whose sums keep the
 // order these bounds have always come from: of this kernel where first-fit
 // layers cover the system, of the plane-streaming kernel where they do not.
-// Measured on the B200, FP64 step: 64-atom LiH, 400 nodes of 33^3 windows,
-// 736 ms all on the plane-streaming kernel, 538 with its long runs there (145
-// to 240 on column pairs alone).
+// Measured on the B200, FP64 step of 64-atom LiH, 400 nodes of 33^3 windows:
+// 400 to 808 ms all on the plane-streaming kernel, 180 (no long run) to 586 with
+// the long runs there, 145 to 240 on column pairs alone.
 //
 // The plane loop is that of sqb_sweep.cuh without the pairs: window vectors of
 // n^3 values, a thread per column and RY adjacent rows, the stencil's planes
