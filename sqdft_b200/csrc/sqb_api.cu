@@ -546,11 +546,12 @@ int prepare_sq_sweep(sqb_ctx *c, const NodeArgs &a, const int *d_list, int count
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
     auto fits = [&](int ry) { return sweep_cols_supported(c->n, c->n_gproj, ry, (size_t)optin); };
     l.redo = c->lay_first_fit && fits(2) ? Redo::Columns : Redo::Plane;
-    if (c->redo_n < count) {  // (a caller's list may name a node more than once)
+    const int ids = std::max(count, c->nnode);  // (a caller's list may name a node more than once)
+    if (c->redo_n < ids) {
       c->redo_n = 0;
       drop_graph(c);  // captured launches hold the old list's address
-      CK(dalloc(&c->d_redo, (size_t)count + 2));  // count, queue head, ids
-      c->redo_n = count;
+      CK(dalloc(&c->d_redo, (size_t)ids + 2));  // count, queue head, ids
+      c->redo_n = ids;
     }
     l.cols = l.s;
     l.cols.ry = c->sweep_ry == 3 && fits(3) ? 3 : 2;

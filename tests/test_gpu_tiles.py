@@ -207,14 +207,11 @@ def test_long_lanczos_runs_keep_the_order_of_their_sums(per_cell, nloc, seed):
         assert _rel(np.asarray(a[k]).reshape(-1), ref[f"{per_cell}_{nloc}_{seed}_{k}"].reshape(-1)) <= 1e-13, k
 
 
-@pytest.mark.parametrize("rows", [0, 3])
-@pytest.mark.parametrize("nloc", [10, 14, 15, 16, 19])
+@pytest.mark.parametrize("nloc,rows", [(n, r) for n in (10, 14, 15, 16, 19) for r in (0, 3) if r == 0 or n <= 16])
 def test_one_column_tile_matches_plane_kernel(nloc, rows):
     """8-atom LiH, where first fit needs four layers, at a stop of 1e-12 Ha, which most runs reach
     late: windows with a warp per row group (up to 31 wide) and with packed columns (from 33 on),
-    n mod 3 of 0, 1 and 2.  The converged bounds agree to the stop and their roundings."""
-    if rows == 3 and nloc > 16:
-        pytest.skip("three rows cover windows up to 33 wide")
+    n mod 3 of 0, 1 and 2 (three rows cover up to 33).  The converged bounds agree to the stop and their roundings."""
     a, b, long = _long_runs(_params("sq", "lih", nloc, cells=1, per_cell=20), 3, rows, 1e-12)
     assert long.any()
     for k in ("chi", "zee"):
@@ -242,3 +239,22 @@ def test_radial_lookup_on_other_grids(grid_kind):
     ref = LocalOracle(grid, loc).charge_density()
     assert np.array_equal(out["b"], ref["b"])
     assert np.array_equal(out["rho_at"], ref["rho_at"])
+
+
+def test_a_list_that_names_long_runs_more_than_once():
+    """sqb_lanczos_moments_nodes with more entries than the block has nodes: the list of nodes to
+    repeat holds them all."""
+    from perf import cases
+    from sqdft_b200 import sq
+
+    c = cases._case(_params("sq", "lih", 12, cells=1, per_cell=14, block="5x4x3", kt=9.0), 2)
+    with sq.Context(c, precision=0) as ctx:
+        ctx.nonlocal_projectors()
+        ctx.set_veff(c.veff)
+        a = ctx.lanczos_moments()
+        long = np.flatnonzero(a["lanczos_iters"].reshape(-1) > 6 * c.nw)
+        nodes = np.concatenate([np.repeat(long, 70), np.arange(c.n_nodes)]).astype(np.int32)
+        b = ctx.lanczos_moments_nodes(nodes)
+    assert long.size and len(nodes) > c.n_nodes + 60
+    for k in ("chi", "zee", "rho_pj", "lanczos_iters"):
+        assert np.array_equal(np.asarray(a[k]).reshape(c.n_nodes, -1)[nodes], np.asarray(b[k]).reshape(len(nodes), -1)), k
